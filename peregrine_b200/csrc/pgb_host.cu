@@ -298,6 +298,8 @@ int build_species(pgb_case *c) {
   if (c->phys.eos != PGB_EOS_CPG) {
     c->sp.tpg = 1;
     RET(fit("cppolyR", c->sp.cppolyR, c->sp.ncp));
+    c->sp.lnT0 = LN_T0;
+    recentre(c->sp.cppolyR, ns, c->sp.ncp, LN_T0);
     RET(fit("hpoly", c->sp.hpoly, c->sp.nh));
   }
   if (c->phys.eos == PGB_EOS_REALGAS || c->phys.eos == PGB_EOS_REALGAS_DF) {

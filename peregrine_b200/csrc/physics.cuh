@@ -22,7 +22,7 @@ struct Species {
   int ns;
   double Ru;
   double Rsp[MAXNS], cp0[MAXNS], h298R[MAXNS], MWinv[MAXNS], hpoly0[MAXNS], h298[MAXNS];
-  double mu0[MAXNS], kappa0[MAXNS], MWqinv[MAXNS], lewis[MAXNS];
+  double mu0[MAXNS], kappa0[MAXNS], MWqinv[MAXNS], lewis[MAXNS], lewisinv[MAXNS];
   double wilkepair[MAXNS * MAXNS];
   double alpha;
   // single-species shortcuts, exact copies of what the per-cell formulas give
@@ -35,6 +35,8 @@ struct Species {
   // peregrine/simulator/mixture/transport/kinetic.py)
   int tpg, kinetic;
   int ncp, nh, nmu, nkappa;
+  // cppolyR's are recentred: coefficients in ln T - lnT0 (recentre)
+  double lnT0;
   double cppolyR[MAXNS * MAXT], hpoly[MAXNS * MAXT], mupoly[MAXNS * MAXT], kappapoly[MAXNS * MAXT];
   // the sub-stepped chemistry's species heat capacities, cp / R_sp in ln T
   // (peregrine/simulator/mixture/eos/base.py:33-47), and molar masses
@@ -77,6 +79,7 @@ inline void species_fill(Species &s, int ns, double alpha, bool constant_transpo
   double *dst[T_NTAB] = {s.Rsp, s.cp0, s.h298R, s.MWinv, s.hpoly0, s.h298, s.mu0, s.kappa0, s.MWqinv, s.lewis};
   for (int q = 0; q < T_NTAB; q++)
     for (int n = 0; n < ns; n++) dst[q][n] = tab[q] ? tab[q][n] : 1.0;
+  for (int n = 0; n < ns; n++) s.lewisinv[n] = 1.0 / s.lewis[n];
   for (int n = 0; n < ns; n++)
     for (int m = 0; m < ns; m++) s.wilkepair[n * MAXNS + m] = wilkepair ? wilkepair[n * ns + m] : 0.25;
   s.R1 = 0.0 + 1.0 * s.Rsp[0];
@@ -89,6 +92,7 @@ inline void species_fill(Species &s, int ns, double alpha, bool constant_transpo
   s.mu1 = s.kappa1 = 0.0;
   s.tpg = s.kinetic = 0;
   s.ncp = s.nh = s.nmu = s.nkappa = 0;
+  s.lnT0 = 0.0;
   s.realgas = s.df = 0;
   if (ns == 1 && constant_transport) {
     volatile double Y = 1.0;
@@ -112,6 +116,24 @@ inline void fit_fill(double *dst, int &nterms, const double *src, int ns, int te
   nterms = terms;
   for (int n = 0; n < ns; n++)
     for (int t = 0; t < MAXT; t++) dst[n * MAXT + t] = t < terms ? src[n * terms + t] : 0.0;
+}
+
+// The fits of cp moved from powers of ln T to powers of ln T - lnT0, the same
+// polynomials.  About ln T = 0 a fit's terms are some 4e4 times their sum
+// (ln T is 5 to 8), so cp and h carried 1e-11 of rounding and T, the root of
+// h(T) - R T, moved by 4e-12 whenever a cell's last bits did; about the
+// middle of the fits' range the terms are the sum's size and so is the
+// rounding.  The move itself cancels as the terms do, hence the wider type.
+constexpr double LN_T0 = 6.9;
+inline void recentre(double *poly, int ns, int terms, double lnT0) {
+  for (int n = 0; n < ns; n++) {
+    long double c[MAXT];
+    for (int t = 0; t < terms; t++) c[t] = poly[n * MAXT + t];
+    // Horner's shift, a coefficient at a time
+    for (int m = 0; m < terms; m++)
+      for (int t = terms - 2; t >= m; t--) c[t] += (long double)lnT0 * c[t + 1];
+    for (int t = 0; t < terms; t++) poly[n * MAXT + t] = (double)c[t];
+  }
 }
 
 // EosState (peregrine/simulator/mixture/eos/base.py:85-86)
@@ -142,44 +164,46 @@ __device__ __forceinline__ void mixmom(YF Y, double &R, double &cp, double &h298
 // the moments of peregrine/simulator/mixture/eos/tpg/model.py:7-9)
 template <int NS, class YF>
 __device__ __forceinline__ void mixmom_tpg(YF Y, double &R, double &h298, double *cc) {
+  // the sums' multiply-adds spelled out: the kernels that form a state then
+  // form the same bits of it, however the compiler arranges each
   R = 0.0, h298 = 0.0;
 #pragma unroll
   for (int t = 0; t < MAXT; t++) cc[t] = 0.0;
   double Ylast = 1.0;
+  auto add = [&](const int n, const double Yn) {
+    R = fma(Yn, kSp.Rsp[n], R);
+    h298 = fma(Yn, kSp.h298R[n], h298);
+#pragma unroll
+    for (int t = 0; t < MAXT; t++)
+      if (t < kSp.ncp) cc[t] = fma(Yn, kSp.cppolyR[n * MAXT + t], cc[t]);
+  };
 #pragma unroll
   for (int n = 0; n < NS - 1; n++) {
     const double Yn = Y(n);
     Ylast -= Yn;
-    R += Yn * kSp.Rsp[n];
-    h298 += Yn * kSp.h298R[n];
-#pragma unroll
-    for (int t = 0; t < MAXT; t++)
-      if (t < kSp.ncp) cc[t] += Yn * kSp.cppolyR[n * MAXT + t];
+    add(n, Yn);
   }
-  R += Ylast * kSp.Rsp[NS - 1];
-  h298 += Ylast * kSp.h298R[NS - 1];
-#pragma unroll
-  for (int t = 0; t < MAXT; t++)
-    if (t < kSp.ncp) cc[t] += Ylast * kSp.cppolyR[(NS - 1) * MAXT + t];
+  add(NS - 1, Ylast);
 }
 
 // ideal_cph: cp and h per mass at T from the moments, h's coefficients built
 // from cp's in the same descent
 // (peregrine/simulator/mixture/caloric/tdepcp/kernels/caloric.mako:4-15)
 __device__ __forceinline__ void ideal_cph(const double *cc, const double h298, const double T, double &cp, double &h) {
-  const double u = log(T);
+  // the antiderivative's recurrence is the same in any shift of ln T
+  const double u = __dsub_rn(log(T), kSp.lnT0);
   cp = 0.0;
   h = 0.0;
   double hcoeff = 0.0;
 #pragma unroll
   for (int m = MAXT - 1; m >= 0; m--) {
     if (m < kSp.ncp) {
-      cp = cp * u + cc[m];
-      hcoeff = cc[m] - (m + 1) * hcoeff;
-      h = h * u + hcoeff;
+      cp = fma(cp, u, cc[m]);
+      hcoeff = fma(-(double)(m + 1), hcoeff, cc[m]);
+      h = fma(h, u, hcoeff);
     }
   }
-  h = h * T + h298;
+  h = fma(h, T, h298);
 }
 
 // fromQ (peregrine/simulator/euler/kernels/state/fromQ.mako:5-19) with the
@@ -203,7 +227,7 @@ __device__ __forceinline__ State fromQ(QF Q, const double Tguess = 0.0) {
     const double tol = 1e5 * 2.220446049250313e-16;
     for (int k = 0; k < 12; k++) {
       ideal_cph(cc, h298, T, cp, h);
-      const double dT = (e - (h - R * T)) / (cp - R);
+      const double dT = (e - fma(-R, T, h)) / (cp - R);
       T += dT;
       if (k >= 2 && fabs(dT) <= tol * T) break;
     }
@@ -253,7 +277,7 @@ __device__ __forceinline__ State frompT(const double p, const double T, YF Y) {
     ideal_cph(cc, h298, T, cp, h);
     s.rho = p / (R * T);
     s.rhoinv = 1.0 / s.rho;
-    s.e = h - R * T;
+    s.e = fma(-R, T, h);
     s.cp = cp;
     s.gamma = cp / (cp - R);
     s.c = sqrt(s.gamma * R * T);
