@@ -44,13 +44,23 @@ __host__ __device__ __forceinline__ long long cell_index(const BlockDev &b, int 
   return (long long)fi + (long long)b.X * ((long long)fj + (long long)b.Y * fk);
 }
 
+// the index in its block of interior cell t, i fastest (a block's cells fit
+// 32 bits: its arrays' component strides do)
+__host__ __device__ __forceinline__ long long inner_cell(const BlockDev &b, long long t) {
+  const unsigned u = (unsigned)t, r = u / (unsigned)b.nx, i = u - r * (unsigned)b.nx;
+  const unsigned k = r / (unsigned)b.ny, j = r - k * (unsigned)b.ny;
+  return cell_index(b, (int)i + NG, (int)j + NG, (int)k + NG);
+}
+
 // The per-cell state of the per-block path, fields of one cell SW apart in
 // vol-strided planes: the EosState (p, T, rhoinv, rho, e, cp, gamma, c), the
 // real gas's root Z, and the double flux's tangent plane of rho e
 // (theta, eps, kappa, zeta[ns - 1]) (peregrine/simulator/mixture/eos/base.py:85-86,
 // realgas/model.py:31-34, realgasdf/model.py:8-10)
 constexpr int SW = 24;
-enum { ST_Z = 8, ST_THETA = 9, ST_EPS = 10, ST_KAPPA = 11, ST_ZETA = 12 };
+// The ideal gases leave the plane's fields unused and, on uniform blocks of the
+// fused passes, keep the cell's velocity at the record's end (uniface.cuh).
+enum { ST_Z = 8, ST_THETA = 9, ST_EPS = 10, ST_KAPPA = 11, ST_ZETA = 12, ST_U = 21 };
 
 // Where a per-block kernel's thread works: its block and its index t in the
 // pass's range over that block.  With a tile table (a packed launch over many
@@ -62,6 +72,37 @@ enum { ST_Z = 8, ST_THETA = 9, ST_EPS = 10, ST_KAPPA = 11, ST_ZETA = 12 };
   const int2 where_ = ctab ? ctab[blockIdx.x] : make_int2(b + (int)blockIdx.y, (int)blockIdx.x); \
   const BlockDev &B = blks[where_.x];                                                                \
   const long long t = (long long)where_.y * blockDim.x + threadIdx.x
+
+// Where a thread of a pass over the faces of all three axes works: RF_TH
+// faces a CTA, the CTAs axis by axis (n0 of axis 0, n1 of axis 1, the rest
+// axis 2), a grid row a block; with tile tables (the three axes' end to end)
+// each 256-face tile is two CTAs.  Returns the axis; the block and the face's
+// number in it in row and t.
+constexpr int RF_TH = 128;
+#ifdef __CUDACC__
+__device__ __forceinline__ int face_work(const unsigned n0, const unsigned n1, const int2 *__restrict__ ctab, int &row,
+                                         unsigned &t) {
+  const unsigned x = blockIdx.x;
+  const int axis = x < n0 ? 0 : x < n0 + n1 ? 1 : 2;
+  if (ctab) {
+    const int2 w = ctab[x >> 1];
+    row = w.x;
+    t = (unsigned)w.y * 256u + (x & 1) * RF_TH + threadIdx.x;
+  } else {
+    row = (int)blockIdx.y;
+    t = (x - (axis == 0 ? 0 : axis == 1 ? n0 : n0 + n1)) * RF_TH + threadIdx.x;
+  }
+  return axis;
+}
+// face t of an axis of a block as the index of the cell on its high side
+__device__ __forceinline__ bool face_cell(const BlockDev &B, const int axis, const unsigned t, long long &R) {
+  const unsigned fx = B.nx + (axis == 0), fy = B.ny + (axis == 1), fz = B.nz + (axis == 2);
+  const unsigned r = t / fx, i = t - r * fx, k = r / fy, j = r - k * fy;
+  if (k >= fz) return false;
+  R = cell_index(B, (int)i + NG, (int)j + NG, (int)k + NG);
+  return true;
+}
+#endif
 
 // one cell of a halo filled from another cell: each side's block start in
 // cells (cv), its cell index inside the block and its component stride

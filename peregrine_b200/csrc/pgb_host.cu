@@ -766,74 +766,118 @@ int build_tiles(pgb_case *c) {
 
 // Each block's uniform form when its metrics allow it: every area vector along
 // its axis alone and equal, the inverse Jacobian diagonal and equal, the cell
-// centres evenly spaced; the representative values are the block's own.
-int detect_uniform(pgb_case *c, bool allow) {
-  const int nb = (int)c->blocks.size();
-  std::vector<double> h;
-  for (int b = 0; b < nb; b++) {
-    HostBlock &HB = c->blocks[b];
-    BlockDev &D = HB.dev;
-    D.uniform = 0;
-    if (!allow) continue;
-    bool ok = true;
-    for (int m = 0; m < PGB_NMETRICS; m++) ok = ok && HB.metrics_set[m];
-    if (!ok) continue;
-    h.resize((size_t)M_NCOMP * D.vol);
-    CK(cudaMemcpy(h.data(), c->d_met + (long long)M_NCOMP * D.cv, sizeof(double) * h.size(), cudaMemcpyDeviceToHost));
-    auto at = [&](int comp, int i, int j, int k) { return h[(size_t)comp * D.vol + cell_index(D, i + NG, j + NG, k + NG)]; };
-    const int n[3] = {D.nx, D.ny, D.nz};
-    auto close = [](double x, double ref, double tol) { return std::fabs(x - ref) <= tol * std::fabs(ref); };
-    double S[3], Jd[3], ex[3], xL[3], xR[3];
-    const double dJ = at(M_DETJINV, 0, 0, 0);
+// centres evenly spaced; the representative values are the block's own.  The
+// metrics are looked over on the device, a cell a thread (they are hundreds
+// of bytes a cell; the host's walk over a copy of them was most of a case's
+// first step), against the block's first cell's.
+struct UniformRef {
+  double dJ, S[3], Jd[3], ex[3], xL[3], xR[3];
+};
+
+__host__ __device__ inline bool uniform_close(double x, double ref, double tol) {
+  return fabs(x - ref) <= tol * fabs(ref);
+}
+
+static __global__ void k_uniform(const BlockDev *__restrict__ blks, const double *__restrict__ met,
+                                 UniformRef *__restrict__ refs, int *__restrict__ bad) {
+  const BlockDev &D = blks[blockIdx.y];
+  const double *h = met + (long long)M_NCOMP * D.cv;
+  const int n[3] = {D.nx, D.ny, D.nz};
+  auto at = [&](int comp, int i, int j, int k) { return h[comp * D.vol + cell_index(D, i + NG, j + NG, k + NG)]; };
+  UniformRef f;
+  f.dJ = at(M_DETJINV, 0, 0, 0);
+  for (int a = 0; a < 3; a++) {
+    const int o[3] = {a == 0 ? -1 : 0, a == 1 ? -1 : 0, a == 2 ? -1 : 0};
+    const double xm = at(M_XCC + a, o[0], o[1], o[2]), x0 = at(M_XCC + a, 0, 0, 0), xf = at(M_XF + 3 * a + a, 0, 0, 0);
+    f.S[a] = at(M_S + 3 * a + a, 0, 0, 0);
+    f.Jd[a] = at(M_JINV + 4 * a, 0, 0, 0);
+    f.ex[a] = x0 - xm, f.xL[a] = xf - xm, f.xR[a] = xf - x0;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) refs[blockIdx.y] = f;
+  bool ok = true;
+  const long long cells = (long long)(n[0] + 2) * (n[1] + 2) * (n[2] + 2);
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < cells; t += (long long)gridDim.x * blockDim.x) {
+    const int i = (int)(t % (n[0] + 2)) - 1, j = (int)((t / (n[0] + 2)) % (n[1] + 2)) - 1,
+              k = (int)(t / ((long long)(n[0] + 2) * (n[1] + 2))) - 1;
+    const int out = (i < 0 || i >= n[0]) + (j < 0 || j >= n[1]) + (k < 0 || k >= n[2]);
+    if (out > 1) continue;
+    // the inverse Jacobian on the first halo layer too
+    for (int a = 0; a < 3; a++)
+      for (int e = 0; e < 3; e++) {
+        const double J = at(M_JINV + 3 * a + e, i, j, k);
+        ok = ok && (a == e ? uniform_close(J, f.Jd[a], 1e-12) : J == 0.0);
+      }
+    if (out) continue;
+    // every interior cell and its low faces
+    ok = ok && uniform_close(at(M_DETJINV, i, j, k), f.dJ, 1e-12);
     for (int a = 0; a < 3; a++) {
-      S[a] = at(M_S + 3 * a + a, 0, 0, 0);
-      Jd[a] = at(M_JINV + 4 * a, 0, 0, 0);
-      int o[3] = {0, 0, 0};
-      o[a] = -1;
-      ex[a] = at(M_XCC + a, 0, 0, 0) - at(M_XCC + a, o[0], o[1], o[2]);
-      xL[a] = at(M_XF + 3 * a + a, 0, 0, 0) - at(M_XCC + a, o[0], o[1], o[2]);
-      xR[a] = at(M_XF + 3 * a + a, 0, 0, 0) - at(M_XCC + a, 0, 0, 0);
+      const int o[3] = {a == 0 ? -1 : 0, a == 1 ? -1 : 0, a == 2 ? -1 : 0};
+      for (int e = 0; e < 3; e++) {
+        const double s = at(M_S + 3 * a + e, i, j, k);
+        ok = ok && (a == e ? uniform_close(s, f.S[a], 1e-12) : s == 0.0);
+        const double d = at(M_XCC + e, i, j, k) - at(M_XCC + e, i + o[0], j + o[1], k + o[2]);
+        ok = ok && (a == e ? uniform_close(d, f.ex[a], 1e-9) : fabs(d) <= 1e-12 * fabs(f.ex[a]));
+      }
     }
-    // every interior cell and its faces; the inverse Jacobian on the first halo layer too
-    for (int k = -1; k <= n[2] && ok; k++)
-      for (int j = -1; j <= n[1] && ok; j++)
-        for (int i = -1; i <= n[0] && ok; i++) {
-          const int out = (i < 0 || i >= n[0]) + (j < 0 || j >= n[1]) + (k < 0 || k >= n[2]);
-          if (out > 1) continue;
-          for (int a = 0; a < 3 && ok; a++)
-            for (int e = 0; e < 3; e++) {
-              const double J = at(M_JINV + 3 * a + e, i, j, k);
-              ok = ok && (a == e ? close(J, Jd[a], 1e-12) : J == 0.0);
-            }
-          if (out) continue;
-          ok = ok && close(at(M_DETJINV, i, j, k), dJ, 1e-12);
-          for (int a = 0; a < 3 && ok; a++) {
-            int o[3] = {0, 0, 0};
-            o[a] = -1;
-            for (int e = 0; e < 3; e++) {
-              const double s = at(M_S + 3 * a + e, i, j, k);
-              ok = ok && (a == e ? close(s, S[a], 1e-12) : s == 0.0);
-              const double d = at(M_XCC + e, i, j, k) - at(M_XCC + e, i + o[0], j + o[1], k + o[2]);
-              ok = ok && (a == e ? close(d, ex[a], 1e-9) : std::fabs(d) <= 1e-12 * std::fabs(ex[a]));
-            }
-          }
-        }
+  }
+  if (!ok) bad[blockIdx.y] = 1;
+}
+
+// the uniform forms of nb blocks (device descriptors d_blks) into dev: their
+// uniform flag and constants; queued on s and waited for
+int uniform_forms(const BlockDev *d_blks, BlockDev *dev, int nb, const double *d_met, double alpha, cudaStream_t s) {
+  if (nb == 0) return PGB_OK;
+  UniformRef *d_ref = nullptr;
+  int *d_bad = nullptr;
+  std::vector<UniformRef> ref(nb);
+  std::vector<int> bad(nb);
+  CK(cudaMallocAsync(&d_ref, sizeof(UniformRef) * nb, s));
+  CK(cudaMallocAsync(&d_bad, sizeof(int) * nb, s));
+  CK(cudaMemsetAsync(d_bad, 0, sizeof(int) * nb, s));
+  for (int b = 0; b < nb; b += 65535) {
+    const int m = std::min(nb - b, 65535);
+    // about eight CTAs an SM in all, each striding over its block
+    k_uniform<<<dim3((unsigned)std::max(1, 8 * 148 / m), (unsigned)m), 256, 0, s>>>(d_blks + b, d_met, d_ref + b,
+                                                                                   d_bad + b);
+  }
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(ref.data(), d_ref, sizeof(UniformRef) * nb, cudaMemcpyDeviceToHost, s));
+  CK(cudaMemcpyAsync(bad.data(), d_bad, sizeof(int) * nb, cudaMemcpyDeviceToHost, s));
+  CK(cudaFreeAsync(d_ref, s));
+  CK(cudaFreeAsync(d_bad, s));
+  CK(cudaStreamSynchronize(s));
+  for (int b = 0; b < nb; b++) {
+    BlockDev &D = dev[b];
+    const UniformRef &f = ref[b];
+    bool ok = !bad[b] && f.dJ > 0.0;
+    for (int a = 0; a < 3; a++) ok = ok && f.S[a] != 0.0 && f.ex[a] != 0.0;
+    D.uniform = ok ? 1 : 0;
     if (!ok) continue;
-    D.uniform = 1;
-    D.detJinv = dJ;
+    D.detJinv = f.dJ;
     for (int a = 0; a < 3; a++) {
-      D.S[a] = S[a], D.Jd[a] = Jd[a], D.ex[a] = ex[a], D.xL[a] = xL[a], D.xR[a] = xR[a];
+      D.S[a] = f.S[a], D.Jd[a] = f.Jd[a], D.ex[a] = f.ex[a], D.xL[a] = f.xL[a], D.xR[a] = f.xR[a];
       // alpha-damping.mako:13-25 on an area vector along axis a
-      const double Sabs = std::sqrt(S[a] * S[a]), Sinv = 1.0 / Sabs;
-      const double nrm = S[a] * Sinv;
-      const double en = ex[a] * nrm;
-      const double dampinv = c->phys.alpha / std::sqrt(en * en);
+      const double Sabs = std::sqrt(f.S[a] * f.S[a]), Sinv = 1.0 / Sabs;
+      const double nrm = f.S[a] * Sinv;
+      const double en = f.ex[a] * nrm;
+      const double dampinv = alpha / std::sqrt(en * en);
       D.damp[a] = dampinv * nrm;
     }
   }
+  return PGB_OK;
+}
+
+int detect_uniform(pgb_case *c) {
   std::vector<BlockDev> devs;
   for (auto &B : c->blocks) devs.push_back(B.dev);
-  CK(cudaMemcpy(c->d_blks, devs.data(), sizeof(BlockDev) * devs.size(), cudaMemcpyHostToDevice));
+  RET(uniform_forms(c->d_blks, devs.data(), (int)devs.size(), c->d_met, c->phys.alpha, c->stream));
+  for (size_t b = 0; b < devs.size(); b++) {
+    for (int m = 0; m < PGB_NMETRICS; m++)
+      if (!c->blocks[b].metrics_set[m]) devs[b].uniform = 0;
+    c->blocks[b].dev = devs[b];
+  }
+  CK(cudaMemcpyAsync(c->d_blks, devs.data(), sizeof(BlockDev) * devs.size(), cudaMemcpyHostToDevice, c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   c->uniform_done = true;
   return PGB_OK;
 }
@@ -1258,6 +1302,22 @@ void mark_cb(void *ctx, int kind) {
   mark(m->c, kind, *m->count);
 }
 
+// how many of the blocks the uniform faces take (uniface.cuh), and the rest:
+// the ideal gases with kepaec, or a Riemann solver on MUSCL's sides, and with
+// Lewis diffusion where viscous; the other forms' faces read the metric arrays
+void uniform_counts(const pgb_physics &p, const Species &sp, const BlockDev *dev, int n, PlainCase &pc) {
+  const bool takes = !sim_df(p.simulator) && (p.eos == PGB_EOS_CPG || p.eos == PGB_EOS_TPG) &&
+                     (p.primary == PGB_FLUX_KEPAEC || p.recon == PGB_RECON_MUSCL) &&
+                     !(sim_visc(p.simulator) && sp.binary);
+  pc.uni = 0;
+  for (int b = 0; b < n; b++) pc.uni += takes && dev[b].uniform;
+  pc.gen = n - pc.uni;
+}
+
+// A case of fewer cells keeps the general passes, a fill a field and a launch
+// an axis: its launch list is held by the tests.
+constexpr long long FEW_CELLS = 2048;
+
 PlainCase plain_case(pgb_case *c, std::vector<BlockDev> &hb) {
   hb.clear();
   for (auto &B : c->blocks) hb.push_back(B.dev);
@@ -1288,10 +1348,15 @@ PlainCase plain_case(pgb_case *c, std::vector<BlockDev> &hb) {
   pc.bcent = c->d_bcent, pc.bcops = c->d_bcops;
   pc.clock = c->d_clock, pc.dt = c->d_dt;
   pc.gensrc = c->gen_src, pc.genmath = c->d_math, pc.blkstride = (int)sizeof(BlockDev);
-  // blocks whose halo is a large share of their cells take the interior cell
-  // pass, where the case's own halo table fills every halo cell (a shard's
-  // traded halo cells get Q alone, so their fields are formed in place)
+  // blocks whose halo is a large share of their cells form the double flux's
+  // state on the interior alone, where the case's own halo table fills every
+  // halo cell (a shard's traded halo cells get Q alone)
+  pc.few = c->interior_cells < FEW_CELLS;
+  pc.fill_all = c->nxrecv == 0 && !pc.few;
   pc.rcell_inner = c->nxrecv == 0 && c->cells > (long long)(1.3 * (double)c->interior_cells) ? 1 : 0;
+  pc.tpg = c->sp.tpg;
+  uniform_counts(c->phys, c->sp, hb.data(), pc.few ? 0 : (int)hb.size(), pc);
+  pc.gen = (int)hb.size() - pc.uni;
   pc.tfrac = 0.0;
   pc.stream = c->stream;
   return pc;
@@ -1451,13 +1516,16 @@ int prepare(pgb_case *c, bool fused) {
     c->form = form;
   }
   // the fused passes read the per-block path's state, transport, gradient
-  // and face arrays and keep the metric arrays' form
-  if (fused && c->form == 2) return ensure_scratch(c);
+  // and face arrays, and the metric arrays of the blocks that are not uniform
+  if (fused && c->form == 2) {
+    if (!c->uniform_done && !sim_df(c->phys.simulator)) RET(detect_uniform(c));
+    return ensure_scratch(c);
+  }
   // the uniform forms are the batched path's alone: the per-block path reads
   // the metric arrays, so a per-block call leaves the detection to the first
   // batched step
   if (fused && !c->uniform_done) {
-    RET(detect_uniform(c, true));
+    RET(detect_uniform(c));
     bool all = true;
     for (auto &B : c->blocks) all = all && B.dev.uniform;
     if (all != c->use_v2) c->tiles_dirty = true;
@@ -2962,8 +3030,8 @@ PlainCase pool_plain(pgb_pool *p, const BlockDev *d_blks, const BlockDev *h_blks
   pc.realgas = p->phys.eos == PGB_EOS_REALGAS || p->phys.eos == PGB_EOS_REALGAS_DF;
   pc.packed = 1;
   pc.dt = p->d_dt;
-  // the pool's blocks are thin (a 1-D domain's halo is most of its cells)
-  pc.rcell_inner = 1;
+  pc.fill_all = 1;
+  pc.gen = n;  // the metric arrays' form for all: most are far below FEW_CELLS
   pc.stream = p->stream;
   return pc;
 }

@@ -31,8 +31,8 @@ __device__ __forceinline__ void rotate3(double *x, const long long st, const dou
 // together, not one round trip each.
 template <int C, bool ROT = true>
 __device__ __forceinline__ void halo_copy(double *__restrict__ base, const int comps, const int vec,
-                                          const double *__restrict__ rots, const long long dcv, const int didx,
-                                          const int dvol, const long long scv, const int sidx, const int svol,
+                                          const double *__restrict__ rots, const long long dcv, const long long didx,
+                                          const int dvol, const long long scv, const long long sidx, const int svol,
                                           const int rot, const int stride) {
   // a block's array starts stride x its cell offset in (its component
   // count, or more where the first comps of wider records are copied)
@@ -688,6 +688,23 @@ __global__ void k_diffflux(const BlockDev *__restrict__ blks, int b, const doubl
   if (DF) Fo[NE * v] += f4;
 }
 
+// The divergence's last step and a combine's terms with their roundings
+// spelled out: the paths form them in kernels of their own, and a compiler
+// free to contract each as it likes would leave their results a last bit apart.
+__device__ __forceinline__ double div_begin(const double faces, const double detJinv) {
+  return __dmul_rn(faces, detJinv);
+}
+__device__ __forceinline__ double div_onto(const double src, const double faces, const double detJinv) {
+  return __fma_rn(faces, detJinv, src);
+}
+__device__ __forceinline__ double term_weight(const double w, const bool step, const double dt) {
+  return step ? __dmul_rn(w, dt) : w;
+}
+__device__ __forceinline__ double term_first(const double w, const double x) { return __dmul_rn(w, x); }
+__device__ __forceinline__ double term_next(const double acc, const double w, const double x) {
+  return __fma_rn(w, x, acc);
+}
+
 // dQ = (low faces - high faces) detJinv (peregrine/simulator/advec/kernels/applyflux.mako:2-11)
 template <int NS>
 __global__ void k_applyflux(const BlockDev *__restrict__ blks, int b, const double *__restrict__ Fi,
@@ -706,8 +723,8 @@ __global__ void k_applyflux(const BlockDev *__restrict__ blks, int b, const doub
   // with append, a source began dQ and the fluxes add to it (applyflux.mako's append)
 #pragma unroll
   for (int l = 0; l < NE; l++) {
-    const double f = (fi[l * v] + fj[l * v] + fk[l * v] - fi[l * v + 1] - fj[l * v + sJ] - fk[l * v + sK]) * detJinv;
-    dQ[l * v] = append ? dQ[l * v] + f : f;
+    const double f = fi[l * v] + fj[l * v] + fk[l * v] - fi[l * v + 1] - fj[l * v + sJ] - fk[l * v + sK];
+    dQ[l * v] = append ? div_onto(dQ[l * v], f, detJinv) : div_begin(f, detJinv);
   }
 }
 
@@ -731,9 +748,9 @@ __global__ void k_applyflux_df(const BlockDev *__restrict__ blks, int b, const d
 #pragma unroll
   for (int l = 0; l < NE; l++) {
     if (l == 4) continue;
-    dQ[l * v] = (fi[l * v] + fj[l * v] + fk[l * v] - fi[l * v + 1] - fj[l * v + sJ] - fk[l * v + sK]) * detJinv;
+    dQ[l * v] = div_begin(fi[l * v] + fj[l * v] + fk[l * v] - fi[l * v + 1] - fj[l * v + sJ] - fk[l * v + sK], detJinv);
   }
-  dQ[4 * v] = (fi[NE * v] + fj[NE * v] + fk[NE * v] - fi[4 * v + 1] - fj[4 * v + sJ] - fk[4 * v + sK]) * detJinv;
+  dQ[4 * v] = div_begin(fi[NE * v] + fj[NE * v] + fk[NE * v] - fi[4 * v + 1] - fj[4 * v + sJ] - fk[4 * v + sK], detJinv);
 }
 
 // one combine (peregrine/integrators/kernels/combine.mako:1-13) on a block's interior
@@ -754,17 +771,17 @@ static __global__ void k_combine(const BlockDev *__restrict__ blks, int b, int n
   const double d = *dt;
   for (int l = 0; l < ne; l++) {
     const long long at = c + l * B.vol;
-    auto term = [&](int n) { return (cd.step && n == cd.nterms - 1) ? cd.w[n] * d * cd.X[n][at] : cd.w[n] * cd.X[n][at]; };
+    auto weight = [&](int n) { return term_weight(cd.w[n], cd.step && n == cd.nterms - 1, d); };
     double acc;
     int n0;
     if (cd.own) {
-      acc = cd.wout * cd.out[at];
+      acc = term_first(cd.wout, cd.out[at]);
       n0 = 0;
     } else {
-      acc = term(0);
+      acc = term_first(weight(0), cd.X[0][at]);
       n0 = 1;
     }
-    for (int n = n0; n < cd.nterms; n++) acc = acc + term(n);
+    for (int n = n0; n < cd.nterms; n++) acc = term_next(acc, weight(n), cd.X[n][at]);
     cd.out[at] = acc;
   }
 }

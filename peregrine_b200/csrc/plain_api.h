@@ -76,9 +76,16 @@ struct PlainCase {
   // exp's tables it reads, and the block record's size
   const void *gensrc, *genmath;
   int blkstride;
-  // the fused passes' cell pass over the interior cells, its fields then
-  // copied into the halo (blocks whose halo is a large share of their cells)
+  // the double flux's passes form the interior's state and copy it into the
+  // halo (blocks whose halo is a large share of their cells)
   int rcell_inner;
+  // the fused passes: blocks whose faces the uniform kernel takes, and the
+  // rest; and whether the interior's fields are formed first and every halo
+  // cell's filled from its source's in one pass (a shard's traded halo cells
+  // get Q alone, so its fields are formed in place)
+  int uni, gen, fill_all;
+  int few;  // a case of few cells: the faces a launch an axis
+  int tpg;  // thermally perfect (else calorically)
   double tfrac;
   cudaStream_t stream;
   void (*mark)(void *ctx, int kind);  // called after each launch, kind 0 halo, 2 block, 4 boundary, 5 CFL

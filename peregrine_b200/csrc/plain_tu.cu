@@ -493,12 +493,12 @@ namespace {
 template <bool VISC>
 void rcell_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
   const RStage &r = *(const RStage *)ctx;
-  k_rcell<NS, VISC><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->tr, pc->hsp, ct);
+  k_rcell<NS, VISC><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->tr, pc->hsp, pc->uni > 0, ct);
 }
 template <bool VISC>
 void rcell_inner_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
   const RStage &r = *(const RStage *)ctx;
-  k_rcell<NS, VISC, true><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->tr, pc->hsp, ct);
+  k_rcell<NS, VISC, true><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->tr, pc->hsp, pc->uni > 0, ct);
 }
 void rsource_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
   const RStage &r = *(const RStage *)ctx;
@@ -508,21 +508,63 @@ void rgrads_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const voi
   const RStage &r = *(const RStage *)ctx;
   k_grads<NS><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->met, pc->grads, 0, ct);
 }
+// the CTAs a block takes of each axis of a pass over every face, and the grid's
+// rows; with tile tables (which lie axis after axis) two CTAs a tile
+bool face_grid(const PlainCase *pc, unsigned *n, unsigned &rows) {
+  rows = pc->ctab[R_FX] ? 1 : (unsigned)pc->nblocks;
+  for (int a = 0; a < 3; a++) {
+    if (pc->ctab[R_FX]) {
+      n[a] = 2 * (unsigned)pc->nctab[R_FX + a];
+    } else {
+      long long most = 0;
+      for (int b = 0; b < pc->nblocks; b++) most = std::max(most, range_size(pc->h_blks[b], R_FX + a));
+      n[a] = (unsigned)((most + RF_TH - 1) / RF_TH);
+    }
+  }
+  return n[0] + n[1] + n[2] > 0 && rows > 0;
+}
+// the uniform blocks' faces of all three axes in one launch
+template <int FN, bool KOREN, bool VISC, bool TPG>
+void ufaces_go(const PlainCase *pc, const RStage *r, int lim) {
+  unsigned n[3], rows;
+  if (!face_grid(pc, n, rows)) return;
+  k_ufaces<NS, FN, KOREN, VISC, TPG><<<dim3(n[0] + n[1] + n[2], rows, 1), UF_TH, 0, pc->stream>>>(
+      pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->F[0], pc->F[1], pc->F[2], lim, n[0], n[1], pc->ctab[R_FX]);
+  mark(pc, 2);
+}
+template <bool VISC, bool TPG>
+void ufaces_launch(const PlainCase *pc, const RStage *r) {
+  const int lim = pc->limiter;
+  switch (pc->primary) {
+    case PGB_FLUX_KEPAEC: ufaces_go<0, false, VISC, TPG>(pc, r, 0); break;
+    case PGB_FLUX_HLLC:
+      if (lim == LIM_KOREN) ufaces_go<FN_HLLC, true, VISC, TPG>(pc, r, lim);
+      else ufaces_go<FN_HLLC, false, VISC, TPG>(pc, r, lim);
+      break;
+    case PGB_FLUX_RUSANOV: ufaces_go<FN_RUSANOV, false, VISC, TPG>(pc, r, lim); break;
+    default: ufaces_go<FN_AUSMUP, false, VISC, TPG>(pc, r, lim); break;
+  }
+}
 }  // namespace
 
 namespace {
-template <int A>
-void rface_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
-  const RStage &r = *(const RStage *)ctx;
+void rface_launch(const PlainCase *pc, const RStage *r, const int only = -1) {
   const int lim = pc->recon == PGB_RECON_MUSCL ? pc->limiter : 0;
+  unsigned n[3], rows;
+  if (!face_grid(pc, n, rows)) return;
+  for (int a = 0; a < 3; a++)
+    if (only >= 0 && a != only) n[a] = 0;
+  const dim3 g(n[0] + n[1] + n[2], rows, 1);
   cudaStream_t s = pc->stream;
-#define PGB_RFACE(FN)                                                                                          \
-  if (pc->visc)                                                                                              \
-    k_rface<NS, A, FN, true><<<g, TH, 0, s>>>(pc->d_blks, b, r.Q, pc->state, pc->tr, pc->hsp, pc->grads,     \
-                                              pc->met, pc->F[A], lim, ct);                                   \
-  else                                                                                                       \
-    k_rface<NS, A, FN, false><<<g, TH, 0, s>>>(pc->d_blks, b, r.Q, pc->state, pc->tr, pc->hsp, pc->grads,    \
-                                               pc->met, pc->F[A], lim, ct);
+#define PGB_RFACE(FN)                                                                                             \
+  if (pc->visc)                                                                                                 \
+    k_rface<NS, FN, true><<<g, RF_TH, 0, s>>>(pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->grads, pc->met, \
+                                              pc->F[0], pc->F[1], pc->F[2], lim, pc->uni > 0, n[0], n[1],       \
+                                              pc->ctab[R_FX]);                                                  \
+  else                                                                                                          \
+    k_rface<NS, FN, false><<<g, RF_TH, 0, s>>>(pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->grads, pc->met, \
+                                               pc->F[0], pc->F[1], pc->F[2], lim, pc->uni > 0, n[0], n[1],      \
+                                               pc->ctab[R_FX]);
   switch (pc->primary) {
     case PGB_FLUX_KEPAEC: PGB_RFACE(0) break;
     case PGB_FLUX_HLLC: PGB_RFACE(FN_HLLC) break;
@@ -530,13 +572,14 @@ void rface_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void
     default: PGB_RFACE(FN_AUSMUP) break;
   }
 #undef PGB_RFACE
+  mark(pc, 2);
 }
 struct RApplyCtx {
   RApplyArgs a;
 };
 void rapply_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
   const RApplyCtx &r = *(const RApplyCtx *)ctx;
-  k_rapply<NS><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, pc->F[0], pc->F[1], pc->F[2], pc->met, r.a, ct);
+  k_rapply<NS><<<dim3(g.x, g.y, NE), TH, 0, pc->stream>>>(pc->d_blks, b, pc->F[0], pc->F[1], pc->F[2], pc->met, r.a, ct);
 }
 struct RCellFluxCtx {
   const double *Q;
@@ -553,7 +596,10 @@ extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs
   // the double flux's interior state pass reads no halo cell: its stage
   // fills Q's halo after that pass, in the state's copy
   const bool df_inner = pc->df && pc->rcell_inner && pc->boxcta && pc->nboxcta > 0;
-  if (!df_inner) {
+  // the other gases likewise: the interior's fields, then Q's halo and every
+  // field's in one pass over the boxes
+  const bool inner = !pc->df && pc->fill_all && pc->boxcta && pc->nboxcta > 0;
+  if (!df_inner && !inner) {
     halo_fill(pc, const_cast<double *>(rs->Q), NE, 1);
     mark(pc, 0);
   }
@@ -592,9 +638,16 @@ extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PGB_OK : cuda_fail(e, "fused double-flux stage");
   }
-  if (pc->rcell_inner) {
-    // the interior cells, then each halo cell's fields from its source's:
-    // the same values, as a halo cell's Q and last T are its source's
+  if (inner) {
+    for_blocks(pc, R_INNER, pc->visc ? rcell_inner_launch<true> : rcell_inner_launch<false>, rs, 8);
+    const HaloFields f{const_cast<double *>(rs->Q), pc->state, pc->tr, pc->hsp, pc->uni > 0, pc->gen > 0,
+                       pc->boxes, pc->boxcta, pc->boxrest, pc->nboxrest, pc->rots};
+    const dim3 g((unsigned)pc->nboxcta, 1, pc->visc ? 3 : 2);
+    if (pc->rots) k_halo_fields<NS, true><<<g, 256, 0, s>>>(f);
+    else k_halo_fields<NS, false><<<g, 256, 0, s>>>(f);
+    mark(pc, 0);
+  } else if (pc->rcell_inner) {
+    // a field's halo at a time
     for_blocks(pc, R_INNER, pc->visc ? rcell_inner_launch<true> : rcell_inner_launch<false>, rs, 8);
     halo_fill(pc, pc->state, 8, HALO_SCALARS, SW);
     mark(pc, 0);
@@ -609,14 +662,22 @@ extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs
   }
   const bool chem = pc->chem == PGB_CHEM_COUPLED;
   if (chem) for_blocks(pc, R_INNER, rsource_launch, rs, 2);
-  if (pc->visc) {
-    for_blocks(pc, R_INNER, rgrads_launch, rs, 2);
-    grads_fill(pc);
-    mark(pc, 0);
+  if (pc->uni > 0) {
+    if (pc->tpg) pc->visc ? ufaces_launch<true, true>(pc, rs) : ufaces_launch<false, true>(pc, rs);
+    else pc->visc ? ufaces_launch<true, false>(pc, rs) : ufaces_launch<false, false>(pc, rs);
   }
-  for_blocks(pc, R_FX, rface_launch<0>, rs, 2);
-  for_blocks(pc, R_FY, rface_launch<1>, rs, 2);
-  for_blocks(pc, R_FZ, rface_launch<2>, rs, 2);
+  if (pc->gen > 0) {
+    if (pc->visc) {
+      // every block's: a block's halo takes its neighbour's, whatever its form
+      for_blocks(pc, R_INNER, rgrads_launch, rs, 2);
+      grads_fill(pc);
+      mark(pc, 0);
+    }
+    if (pc->few)
+      for (int a = 0; a < 3; a++) rface_launch(pc, rs, a);
+    else
+      rface_launch(pc, rs);
+  }
   RApplyCtx ra{};
   RApplyArgs &a = ra.a;
   a.dQ = rs->dQ;

@@ -43,6 +43,7 @@
 #include "physics.cuh"
 #include "plain.cuh"
 #include "plain_api.h"
+#include "uniface.cuh"
 
 namespace pgb {
 
@@ -53,15 +54,13 @@ template <int NS, bool VISC, bool INNER = false>
 __global__ void __launch_bounds__(256) k_rcell(const BlockDev *__restrict__ blks, int b,
                                                const double *__restrict__ Qall, double *__restrict__ stall,
                                                double *__restrict__ trall, double *__restrict__ hall,
-                                               const int2 *__restrict__ ctab = nullptr) {
+                                               const int uvel, const int2 *__restrict__ ctab = nullptr) {
   constexpr int NE = 4 + NS;
   PGB_WHERE(B, tt);
   long long t = tt;
   if (INNER) {
     if (tt >= (long long)B.nx * B.ny * B.nz) return;
-    const int i = (int)(tt % B.nx) + NG, j = (int)((tt / B.nx) % B.ny) + NG;
-    const int k = (int)(tt / ((long long)B.nx * B.ny)) + NG;
-    t = cell_index(B, i, j, k);
+    t = inner_cell(B, tt);
   } else if (t >= B.vol) {
     return;
   }
@@ -72,6 +71,11 @@ __global__ void __launch_bounds__(256) k_rcell(const BlockDev *__restrict__ blks
   const State s = fromQ<NS>(Qf, st[1 * v]);
   st[0 * v] = s.p, st[1 * v] = s.T, st[2 * v] = s.rhoinv, st[3 * v] = s.rho;
   st[4 * v] = s.e, st[5 * v] = s.cp, st[6 * v] = s.gamma, st[7 * v] = s.c;
+  if (uvel) {
+    // the velocity the uniform faces read (uniface.cuh)
+#pragma unroll
+    for (int m = 0; m < 3; m++) st[(ST_U + m) * v] = Qf(1 + m) * s.rhoinv;
+  }
   if (VISC) {
     double tr[2 + NS], h[NS];
     transport<NS, decltype(Qf), false>(Qf, s, tr, h, 0.0);
@@ -113,32 +117,45 @@ __device__ __forceinline__ void rface(const BlockDev &B, const double *Q, const 
   }
 }
 
-// One face a thread over a pass's faces of axis A: the advective flux and,
-// with VISC, the diffusive rows in the same thread, stored once (the
-// per-block path's k_riemann then k_diffflux, without the flux's round trip
-// between them)
-template <int NS, int A, int FN, bool VISC>
-__global__ void __launch_bounds__(256, 2) k_rface(const BlockDev *__restrict__ blks, int b, const double *__restrict__ Qall,
-                                               const double *__restrict__ stall, const double *__restrict__ trall,
-                                               const double *__restrict__ hall, const double *__restrict__ gall,
-                                               const double *__restrict__ met, double *__restrict__ Fall, const int lim,
-                                               const int2 *__restrict__ ctab = nullptr) {
+// One face a thread: the advective flux and, with VISC, the diffusive rows in
+// the same thread, stored once (the per-block path's k_riemann then
+// k_diffflux, without the flux's round trip between them).  All three axes'
+// faces in one launch, the CTAs of an axis together: no axis waits for the
+// last CTAs of the one before, which on small cases is most of a pass
+template <int NS, int FN, bool VISC>
+__global__ void __launch_bounds__(RF_TH, 4) k_rface(const BlockDev *__restrict__ blks, const double *__restrict__ Qall,
+                                                  const double *__restrict__ stall, const double *__restrict__ trall,
+                                                  const double *__restrict__ hall, const double *__restrict__ gall,
+                                                  const double *__restrict__ met, double *F0, double *F1, double *F2,
+                                                  const int lim, const int skipu, const unsigned n0, const unsigned n1,
+                                                  const int2 *__restrict__ ctab) {
   constexpr int NE = 4 + NS, NGRAD = NE - 1;
-  PGB_WHERE(B, t);
-  int i, j, k;
-  if (!face_at<A>(B, t, i, j, k)) return;
-  const long long R = cell_index(B, i, j, k);
+  unsigned t;
+  int row;
+  const int axis = face_work(n0, n1, ctab, row, t);
+  const BlockDev &B = blks[row];
+  // the uniform blocks' faces are k_ufaces'
+  if (skipu && B.uniform) return;
+  long long R;
+  if (!face_cell(B, axis, t, R)) return;
   double F[NE];
-  rface<NS, A, FN, VISC>(B, Qall + NE * B.cv, stall + SW * B.cv, VISC ? trall + (2 + NS) * B.cv : nullptr,
-                         VISC ? hall + NS * B.cv : nullptr, VISC ? gall + 3 * NGRAD * B.cv : nullptr,
-                         met + M_NCOMP * B.cv, lim, R, F);
-  double *Fo = Fall + NE * B.cv + R;
+  const double *Q = Qall + NE * B.cv, *st = stall + SW * B.cv, *M = met + M_NCOMP * B.cv;
+  const double *tr = VISC ? trall + (2 + NS) * B.cv : nullptr, *hs = VISC ? hall + NS * B.cv : nullptr;
+  const double *gr = VISC ? gall + 3 * NGRAD * B.cv : nullptr;
+  if (axis == 0) rface<NS, 0, FN, VISC>(B, Q, st, tr, hs, gr, M, lim, R, F);
+  else if (axis == 1) rface<NS, 1, FN, VISC>(B, Q, st, tr, hs, gr, M, lim, R, F);
+  else rface<NS, 2, FN, VISC>(B, Q, st, tr, hs, gr, M, lim, R, F);
+  double *Fo = (axis == 0 ? F0 : axis == 1 ? F1 : F2) + NE * B.cv + R;
 #pragma unroll
   for (int l = 0; l < NE; l++) Fo[l * B.vol] = F[l];
 }
 
-// The divergence of each interior cell added to its source (the per-block
-// applyflux's order) and the stage's combines, dQ kept in the thread
+// The divergence added to the source (the per-block applyflux's order) and the
+// stage's combines, a component of a cell a thread (the grid's plane the
+// component).  A thread's nine loads are in flight at once and a launch has NE
+// times the threads of a cell-a-thread pass, which walked the components one
+// after another: 64^3 of nine species 65 us and a latency-bound 37 x 29 x 23
+// of the same 32 us that way (ncu).
 template <int NS>
 __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blks, int b, const double *__restrict__ Fi,
                                                 const double *__restrict__ Fj, const double *__restrict__ Fk,
@@ -147,33 +164,35 @@ __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blk
   constexpr int NE = 4 + NS;
   PGB_WHERE(B, t);
   if (t >= (long long)B.nx * B.ny * B.nz) return;
-  const int i = (int)(t % B.nx) + NG, j = (int)((t / B.nx) % B.ny) + NG, k = (int)(t / ((long long)B.nx * B.ny)) + NG;
-  const long long c = cell_index(B, i, j, k), v = B.vol;
+  const long long c = inner_cell(B, t), v = B.vol;
   const long long sJ = B.X, sK = (long long)B.X * B.Y;
-  const double detJinv = met[M_NCOMP * B.cv + M_DETJINV * v + c];
-  const double *fi = Fi + NE * B.cv + c, *fj = Fj + NE * B.cv + c, *fk = Fk + NE * B.cv + c;
-  const long long at = NE * B.cv + c;
+  const long long at = NE * B.cv + (int)blockIdx.z * v + c;
+  const double *fi = Fi + at, *fj = Fj + at, *fk = Fk + at;
+  const double detJinv = B.uniform ? B.detJinv : met[M_NCOMP * B.cv + M_DETJINV * v + c];
   const double dt = *a.dt;
-  double first[NE];
+  double x[2][4];
 #pragma unroll
-  for (int l = 0; l < NE; l++) {
-    const double f = (fi[l * v] + fj[l * v] + fk[l * v] - fi[l * v + 1] - fj[l * v + sJ] - fk[l * v + sK]) * detJinv;
-    const double dq = a.chem ? a.dQ[at + l * v] + f : f;
-    if (a.write_dq) a.dQ[at + l * v] = dq;
-    for (int m = 0; m < a.ncomb; m++) {
-      const RCombine &cb = a.comb[m];
-      auto val = [&](int n) {
-        const int s = cb.src[n];
-        return s == -1 ? dq : s == -2 ? first[l] : cb.X[n][at + l * v];
-      };
-      auto term = [&](int n) {
-        return (cb.step && n == cb.nterms - 1) ? cb.w[n] * dt * val(n) : cb.w[n] * val(n);
-      };
-      double acc = term(0);
-      for (int n = 1; n < cb.nterms; n++) acc = acc + term(n);
-      if (m == 0) first[l] = acc;
-      if (cb.write) cb.out[at + l * v] = acc;
-    }
+  for (int m = 0; m < 2; m++)
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+      x[m][n] = m < a.ncomb && n < a.comb[m].nterms && a.comb[m].src[n] >= 0 ? a.comb[m].X[n][at] : 0.0;
+  const double src = a.chem ? a.dQ[at] : 0.0;
+  const double f = fi[0] + fj[0] + fk[0] - fi[1] - fj[sJ] - fk[sK];
+  const double dq = a.chem ? div_onto(src, f, detJinv) : div_begin(f, detJinv);
+  if (a.write_dq) a.dQ[at] = dq;
+  double first = 0.0;
+#pragma unroll
+  for (int m = 0; m < 2; m++) {
+    if (m >= a.ncomb) break;
+    const RCombine &cb = a.comb[m];
+    auto val = [&](const int n) { return cb.src[n] == -1 ? dq : cb.src[n] == -2 ? first : x[m][n]; };
+    auto weight = [&](const int n) { return term_weight(cb.w[n], cb.step && n == cb.nterms - 1, dt); };
+    double acc = term_first(weight(0), val(0));
+#pragma unroll
+    for (int n = 1; n < 4; n++)
+      if (n < cb.nterms) acc = term_next(acc, weight(n), val(n));
+    if (m == 0) first = acc;
+    if (cb.write) cb.out[at] = acc;
   }
 }
 
@@ -244,7 +263,7 @@ __global__ void __launch_bounds__(256) k_rcellflux_df(const BlockDev *__restrict
   double first[NE];
 #pragma unroll
   for (int l = 0; l < NE; l++) {
-    const double dq = acc[l] * detJinv;
+    const double dq = div_begin(acc[l], detJinv);
     if (a.write_dq) a.dQ[at + l * v] = dq;
     for (int m = 0; m < a.ncomb; m++) {
       const RCombine &cb = a.comb[m];
@@ -252,11 +271,9 @@ __global__ void __launch_bounds__(256) k_rcellflux_df(const BlockDev *__restrict
         const int s = cb.src[n];
         return s == -1 ? dq : s == -2 ? first[l] : cb.X[n][at + l * v];
       };
-      auto term = [&](int n) {
-        return (cb.step && n == cb.nterms - 1) ? cb.w[n] * dt * val(n) : cb.w[n] * val(n);
-      };
-      double acc = term(0);
-      for (int n = 1; n < cb.nterms; n++) acc = acc + term(n);
+      auto weight = [&](int n) { return term_weight(cb.w[n], cb.step && n == cb.nterms - 1, dt); };
+      double acc = term_first(weight(0), val(0));
+      for (int n = 1; n < cb.nterms; n++) acc = term_next(acc, weight(n), val(n));
       if (m == 0) first[l] = acc;
       if (cb.write) cb.out[at + l * v] = acc;
     }
@@ -293,11 +310,9 @@ __global__ void __launch_bounds__(256) k_reactors(const ReactorStage a) {
         const int src = cb.src[n];
         return src == -1 ? dq : src == -2 ? first[l] : cb.X[n][at];
       };
-      auto term = [&](int n) {
-        return (cb.step && n == cb.nterms - 1) ? cb.w[n] * dt * val(n) : cb.w[n] * val(n);
-      };
-      double acc = term(0);
-      for (int n = 1; n < cb.nterms; n++) acc = acc + term(n);
+      auto weight = [&](int n) { return term_weight(cb.w[n], cb.step && n == cb.nterms - 1, dt); };
+      double acc = term_first(weight(0), val(0));
+      for (int n = 1; n < cb.nterms; n++) acc = term_next(acc, weight(n), val(n));
       if (m == 0) first[l] = acc;
       if (cb.write) cb.out[at] = acc;
     }
@@ -367,9 +382,9 @@ __global__ void __launch_bounds__(256) k_reactors_warp(const ReactorStage a) {
       const int src = cb.src[n];
       return src == -1 ? dq : src == -2 ? first : cb.X[n][at];
     };
-    auto term = [&](int n) { return (cb.step && n == cb.nterms - 1) ? cb.w[n] * dt * val(n) : cb.w[n] * val(n); };
-    double acc = term(0);
-    for (int n = 1; n < cb.nterms; n++) acc = acc + term(n);
+    auto weight = [&](int n) { return term_weight(cb.w[n], cb.step && n == cb.nterms - 1, dt); };
+    double acc = term_first(weight(0), val(0));
+    for (int n = 1; n < cb.nterms; n++) acc = term_next(acc, weight(n), val(n));
     if (m == 0) first = acc;
     if (cb.write) cb.out[at] = acc;
   }

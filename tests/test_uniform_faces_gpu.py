@@ -1,0 +1,93 @@
+"""The fused passes' faces on uniform blocks (csrc/uniface.cuh) and the passes
+around them (every field's halo in one pass, the divergence and combines a
+component a thread) against the per-block path, at extents where a face range
+ends inside a CTA, a block is two cells thin, or blocks of one case differ in
+form.
+
+The bar: both paths round each flux within a few eps of its own size, the
+largest the pressure's in a momentum row and the enthalpy's in the energy row,
+some 10 eps each of a face; over three steps of a CFL number below one a row
+moves by at most that, 1e-12 of its largest value being some 4000 eps."""
+
+import numpy as np
+import pytest
+
+from peregrine_b200 import cases, native
+from peregrine_b200.mesher import CubeMesher
+
+pytestmark = pytest.mark.gpu
+
+
+def pair(cfg_of, mesh_of, prims_of, dt, steps=3):
+    import peregrine_b200 as pg
+
+    out = []
+    for launch in ("batched", "per-block"):
+        cfg, mesh = cfg_of(launch), mesh_of()
+        mb = pg.get_solver(cfg, mesh, pg.get_backend("cuda", cfg))
+        mb.set_prims(prims_of(mb))
+        mb.step(dt, steps)
+        out.append(mb)
+    return out
+
+
+def compare(a, b, bar=1e-12):
+    assert a.path == native.PATH_BATCHED and b.path == native.PATH_PER_BLOCK
+    for x, y in zip(a.blocks, b.blocks):
+        got, want = x.Q.get()[x.mesh.interior], y.Q.get()[y.mesh.interior]
+        scale = np.abs(want).reshape(-1, want.shape[-1]).max(axis=0)
+        scale[1:4] = scale[1:4].max()
+        scale[scale == 0.0] = 1.0
+        err = (np.abs(got - want).reshape(-1, want.shape[-1]).max(axis=0) / scale).max()
+        assert err < bar, err
+
+
+def box(cells, blocks=(1, 1, 1), lengths=(2 * np.pi,) * 3, jostle=0.0):
+    cuts = [[n // b + (1 if m < n - n // b * b else 0) for m in range(b)] for n, b in zip(cells, blocks)]
+    return CubeMesher(mbdims=list(blocks), cells=cuts, lengths=list(lengths), periodic=[True] * 3, jostle=jostle)
+
+
+@pytest.mark.parametrize("cells,blocks", [((13, 17, 11), (1, 1, 1)), ((2, 33, 35), (1, 1, 1)), ((37, 2, 31), (1, 1, 1)),
+                                          ((64, 16, 2), (2, 1, 1)), ((19, 16, 21), (2, 2, 3))])
+@pytest.mark.parametrize("primary,recon,limiter", [("kepaec", "constant", None), ("hllc", "muscl", "koren"),
+                                                   ("hllc", "muscl", "vanleer"), ("rusanov", "muscl", "minmod"),
+                                                   ("ausmup", "muscl", "mc")])
+def test_calorically_perfect(cells, blocks, primary, recon, limiter):
+    for simulator, ns in (("navier-stokes", 3), ("euler", 2)):
+        a, b = pair(lambda launch: cases.mixing_config(simulator, "tvd-rk3", primary, recon, limiter, ns, launch),
+                    lambda: box(cells, blocks), lambda mb: cases.rough_prims(mb.metrics, ns, seed=3, speed=200.0), 1e-5)
+        compare(a, b)
+
+
+@pytest.mark.parametrize("cells,blocks", [((13, 17, 11), (1, 1, 1)), ((23, 10, 16), (2, 1, 2))])
+@pytest.mark.parametrize("tables,primary,recon,limiter", [("h2o2_gri30", "hllc", "muscl", "koren"),
+                                                          ("h2o2_gri30", "kepaec", "constant", None),
+                                                          ("h2o2_gri30", "rusanov", "muscl", "superbee")])
+def test_thermally_perfect(cells, blocks, tables, primary, recon, limiter):
+    def prims(mb):
+        MW = mb.mixture.constants()["MW"]
+        return cases.reacting_prims(mb.metrics, mb.mixture.spnames, MW, cells[0], seed=5, width=2.0, dT=500.0,
+                                    radicals=1e-3)
+
+    a, b = pair(lambda launch: cases.reacting_config("navier-stokes", "tvd-rk3", primary, recon, limiter, True, tables,
+                                                     launch),
+                lambda: box(cells, blocks, (0.01,) * 3), prims, 2e-8)
+    # T's root carries the fits' rounding, 1e-13 of T, into the pressure, whose
+    # difference across a cell drives a momentum a thousandth of its flux
+    compare(a, b, 1e-11)
+
+
+def test_uniform_and_curvilinear_blocks_in_one_case():
+    # a jostled block is read by its metric arrays, a lattice one is not; the
+    # faces between them are formed by both
+    class Half(CubeMesher):
+        def _shape(self, blk, ijk):
+            self.jostle = 0.1 if ijk[0] else 0.0
+            super()._shape(blk, ijk)
+
+    def mesh():
+        return Half(mbdims=[2, 1, 1], cells=[[13, 12], [14], [11]], lengths=[2 * np.pi] * 3, periodic=[True] * 3)
+
+    a, b = pair(lambda launch: cases.mixing_config("navier-stokes", "tvd-rk3", "hllc", "muscl", "koren", 2, launch),
+                mesh, lambda mb: cases.rough_prims(mb.metrics, 2, seed=3, speed=200.0), 1e-5)
+    compare(a, b)
