@@ -140,6 +140,9 @@ struct pgb_case {
   HaloPatch *d_boxes = nullptr;
   int2 *d_boxcta = nullptr;
   HaloEntry *d_boxrest = nullptr;
+  HaloPatch *d_boxes0 = nullptr;  // the first face layer (the gradients' fill)
+  int2 *d_boxcta0 = nullptr;
+  long long nboxcta0 = 0;
   long long nboxcta = 0, nboxrest = 0;
   // the rotationally periodic faces' rotations, then the products a halo
   // cell reached across two of them needs, 3 x 3 each
@@ -156,6 +159,9 @@ struct pgb_case {
   size_t fused_smem = 0;
   bool tiles_dirty = true;
   bool uniform_done = false;
+  void *d_uref = nullptr;  // the blocks' first cells' metrics (UniformRef) and where a block differs from them
+  int *d_ubad = nullptr;
+  bool by_passes = false;  // form 1 stepping by the fused passes (passes_take)
   bool use_v2 = false;  // every block uniform: the uniform-metric fused kernel
   int form = 0;         // the batched path's form: 1 the fused stage kernel, 2 the fused passes
   // a shard's exchange with the other ranks' blocks: the cells it packs and
@@ -583,7 +589,7 @@ void build_halo(pgb_case *c, std::vector<HaloEntry> &out, long long &n_l0, std::
 // source and the source index is affine in the cell's (a face whose
 // neighbour is at least NG cells thick, an edge line along a block); the
 // cells of any other box are listed one by one in rest.
-void build_boxes(pgb_case *c, std::vector<HaloPatch> &boxes, std::vector<HaloEntry> &rest) {
+void build_boxes(pgb_case *c, std::vector<HaloPatch> &boxes, std::vector<HaloEntry> &rest, bool first = false) {
   boxes.clear();
   rest.clear();
   auto box = [&](int b, const int lo[3], const int hi[3]) {
@@ -643,11 +649,12 @@ void build_boxes(pgb_case *c, std::vector<HaloPatch> &boxes, std::vector<HaloEnt
     for (int f = 0; f < 6; f++) {
       const int a = f / 2;
       int lo[3] = {0, 0, 0}, hi[3] = {n[0], n[1], n[2]};
-      lo[a] = f % 2 == 0 ? -NG : n[a];
-      hi[a] = lo[a] + NG;
+      const int depth = first ? 1 : NG;
+      lo[a] = f % 2 == 0 ? -depth : n[a];
+      hi[a] = lo[a] + depth;
       box(b, lo, hi);
     }
-    for (int a = 0; a < 3; a++) {
+    for (int a = 0; a < 3 && !first; a++) {
       const int a1 = (a + 1) % 3, a2 = (a + 2) % 3;
       for (int s1 = 0; s1 < 2; s1++)
         for (int s2 = 0; s2 < 2; s2++) {
@@ -709,13 +716,43 @@ const V2Inst kV2[] = {PGB_V2(256, 1, 24, 7), PGB_V2(256, 1, 30, 6), PGB_V2(128, 
 #undef PGB_V3
 constexpr int kNV2 = sizeof(kV2) / sizeof(kV2[0]);
 
-// the uniform kernel's default tile: i and j cut evenly in pieces the layout holds
-void default_tile2(HostBlock &B, const V2Inst &v) {
+// the uniform kernel's default tile: i and j cut evenly in pieces the layout
+// holds, k in ksplit runs
+void default_tile2(HostBlock &B, const V2Inst &v, int ksplit) {
   const int pi = (B.nx + v.tw - 1) / v.tw;
   const int pj = (B.ny + v.th - 1) / v.th;
   B.tw = (B.nx + pi - 1) / pi;
   B.th = (B.ny + pj - 1) / pj;
-  B.kchunk = (B.nz + 2) / 3;
+  B.kchunk = (B.nz + ksplit - 1) / ksplit;
+}
+
+// The runs the default tiles cut k in: the fewest rounds of CTAs over the
+// device's SMs times the planes a tile marches, its own and the TILE_LEAD it
+// reads before its first (measured with the launch at 2.1 us a plane and 9 us
+// over them: 32^3 in 3 runs 0.130 ms an RK4 step, in 11 0.062, in 16, more
+// tiles than SMs, 0.082; 64^3 in 3 runs 0.263, in 4 0.204, in 5 0.214; the
+// 27-block 128^3 in 1, 2, 3 and 4 runs 1.318, 1.213, 1.317 and 1.321).
+constexpr int TILE_LEAD = 4;
+int default_ksplit(const pgb_case *c) {
+  const V2Inst &v = kV2[c->v2];
+  int dev = 0, sms = 148, nzmax = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long slots = (long long)sms * v.minb;
+  for (const HostBlock &B : c->blocks) nzmax = std::max(nzmax, B.nz);
+  int best = 1;
+  long long least = 0;
+  for (int s = 1; s <= std::min(nzmax, 32); s++) {
+    long long tiles = 0, most = 0;
+    for (const HostBlock &B : c->blocks) {
+      const long long kc = (B.nz + s - 1) / s;
+      tiles += (long long)((B.nx + v.tw - 1) / v.tw) * ((B.ny + v.th - 1) / v.th) * ((B.nz + kc - 1) / kc);
+      most = std::max(most, kc);
+    }
+    const long long cost = (tiles + slots - 1) / slots * (most + TILE_LEAD);
+    if (s == 1 || cost < least) best = s, least = cost;
+  }
+  return best;
 }
 
 bool tile_fits(const pgb_case *c, int tw, int th) {
@@ -727,10 +764,11 @@ int build_tiles(pgb_case *c) {
   std::vector<TileDev> tiles;
   size_t smem = 0;
   const bool visc = c->phys.simulator == PGB_NAVIER_STOKES;
+  const int ksplit = c->use_v2 ? default_ksplit(c) : 1;
   for (int b = 0; b < (int)c->blocks.size(); b++) {
     HostBlock &B = c->blocks[b];
     if (B.tw <= 0 || !tile_fits(c, B.tw, B.th)) {
-      if (c->use_v2) default_tile2(B, kV2[c->v2]);
+      if (c->use_v2) default_tile2(B, kV2[c->v2], ksplit);
       else default_tile(B);
     }
     const size_t need = !c->use_v2 ? fused_smem(B.tw, B.th, visc) : visc ? kV2[c->v2].smvisc : kV2[c->v2].smeuler;
@@ -825,14 +863,10 @@ static __global__ void k_uniform(const BlockDev *__restrict__ blks, const double
 
 // the uniform forms of nb blocks (device descriptors d_blks) into dev: their
 // uniform flag and constants; queued on s and waited for
-int uniform_forms(const BlockDev *d_blks, BlockDev *dev, int nb, const double *d_met, double alpha, cudaStream_t s) {
-  if (nb == 0) return PGB_OK;
-  UniformRef *d_ref = nullptr;
-  int *d_bad = nullptr;
+int uniform_forms(const BlockDev *d_blks, BlockDev *dev, int nb, const double *d_met, double alpha, UniformRef *d_ref,
+                  int *d_bad, cudaStream_t s) {
   std::vector<UniformRef> ref(nb);
   std::vector<int> bad(nb);
-  CK(cudaMallocAsync(&d_ref, sizeof(UniformRef) * nb, s));
-  CK(cudaMallocAsync(&d_bad, sizeof(int) * nb, s));
   CK(cudaMemsetAsync(d_bad, 0, sizeof(int) * nb, s));
   for (int b = 0; b < nb; b += 65535) {
     const int m = std::min(nb - b, 65535);
@@ -843,8 +877,6 @@ int uniform_forms(const BlockDev *d_blks, BlockDev *dev, int nb, const double *d
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(ref.data(), d_ref, sizeof(UniformRef) * nb, cudaMemcpyDeviceToHost, s));
   CK(cudaMemcpyAsync(bad.data(), d_bad, sizeof(int) * nb, cudaMemcpyDeviceToHost, s));
-  CK(cudaFreeAsync(d_ref, s));
-  CK(cudaFreeAsync(d_bad, s));
   CK(cudaStreamSynchronize(s));
   for (int b = 0; b < nb; b++) {
     BlockDev &D = dev[b];
@@ -870,7 +902,8 @@ int uniform_forms(const BlockDev *d_blks, BlockDev *dev, int nb, const double *d
 int detect_uniform(pgb_case *c) {
   std::vector<BlockDev> devs;
   for (auto &B : c->blocks) devs.push_back(B.dev);
-  RET(uniform_forms(c->d_blks, devs.data(), (int)devs.size(), c->d_met, c->phys.alpha, c->stream));
+  RET(uniform_forms(c->d_blks, devs.data(), (int)devs.size(), c->d_met, c->phys.alpha, (UniformRef *)c->d_uref,
+                    c->d_ubad, c->stream));
   for (size_t b = 0; b < devs.size(); b++) {
     for (int m = 0; m < PGB_NMETRICS; m++)
       if (!c->blocks[b].metrics_set[m]) devs[b].uniform = 0;
@@ -993,6 +1026,10 @@ int build_plans(pgb_case *c) {
 }
 
 int grid_for(long long n, int threads) { return (int)std::max<long long>(1, (n + threads - 1) / threads); }
+
+// A case of fewer cells keeps the general passes, a fill a field and a launch
+// an axis: its launch list is held by the tests.
+constexpr long long FEW_CELLS = 2048;
 
 enum { K_HALO = 0, K_FUSED = 1, K_BLOCK = 2, K_COMBINE = 3 };
 
@@ -1181,6 +1218,9 @@ int cfl_prologue(pgb_case *c, int qphys, int &count) {
   return PGB_OK;
 }
 
+// whether the batched path's stages are the fused passes
+bool passes(const pgb_case *c) { return c->form == 2 || (c->form == 1 && c->by_passes); }
+
 // one stage of the fused passes (react.cuh): the plan's combines on physical
 // registers; with dq set (a right-hand side alone) no combine, dQ stored there
 int launch_react(pgb_case *c, const FusedStagePlan &p, int &count, int dq = -1) {
@@ -1206,7 +1246,7 @@ int launch_react(pgb_case *c, const FusedStagePlan &p, int &count, int dq = -1) 
   pc.mark = mark_cb;
   pc.ctx = &mc;
   pc.packed = 1;
-  c->state_stale = false;
+  c->state_stale = c->form != 2;  // form 1 keeps no state array, whichever way it steps
   return kPlain[c->phys.ns - 1].fused(&pc, &r);
 }
 
@@ -1226,7 +1266,7 @@ int step_fused(pgb_case *c, int &count) {
   }
   CK(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned int) * plan.size(), c->stream));
   for (int s = 0; s < (int)plan.size(); s++)
-    RET(c->form == 2 ? launch_react(c, plan[s], count) : launch_fused(c, plan[s], s, count));
+    RET(passes(c) ? launch_react(c, plan[s], count) : launch_fused(c, plan[s], s, count));
   if (c->ctrl_cfl) {
     k_clock<<<1, 1, 0, c->stream>>>(c->d_clock, c->d_dt);
     mark(c, K_COMBINE, count);
@@ -1241,7 +1281,7 @@ int step_fused(pgb_case *c, int &count) {
 // other weights zero), so it writes exactly the dQ it forms.  The halo fill
 // of q comes first, as in a stage.
 int rhs_fused(pgb_case *c, int qphys, int dqphys, int &count) {
-  if (c->form == 2) {
+  if (passes(c)) {
     FusedStagePlan p{};
     p.qin = qphys;
     return launch_react(c, p, count, dqphys);
@@ -1314,9 +1354,6 @@ void uniform_counts(const pgb_physics &p, const Species &sp, const BlockDev *dev
   pc.gen = n - pc.uni;
 }
 
-// A case of fewer cells keeps the general passes, a fill a field and a launch
-// an axis: its launch list is held by the tests.
-constexpr long long FEW_CELLS = 2048;
 
 PlainCase plain_case(pgb_case *c, std::vector<BlockDev> &hb) {
   hb.clear();
@@ -1332,6 +1369,7 @@ PlainCase plain_case(pgb_case *c, std::vector<BlockDev> &hb) {
   pc.nhalo = c->nhalo, pc.nhalo_l0 = c->nhalo_l0;
   pc.boxes = c->d_boxes, pc.boxcta = c->d_boxcta, pc.nboxcta = c->nboxcta;
   pc.boxrest = c->d_boxrest, pc.nboxrest = c->nboxrest;
+  pc.boxes0 = c->d_boxes0, pc.boxcta0 = c->d_boxcta0, pc.nboxcta0 = c->nboxcta0;
   pc.rots = c->d_rots;
   pc.visc = sim_visc(c->phys.simulator);
   pc.packed = c->packed ? 1 : 0;
@@ -1507,6 +1545,21 @@ int build_bcs(pgb_case *c) {
   return PGB_OK;
 }
 
+// Whether the single-species kepaec case (form 1) steps by the fused passes
+// where its grid is not uniform: 64^3 in four blocks, a Navier-Stokes RK4 step
+// 0.46 ms against the general stage kernel's 1.85 ms.  The stage kernel
+// keeps the cases of few cells, a shard (its gradients come of Q's traded
+// halo) and a case whose passes' arrays do not fit the device beside it.
+bool passes_take(pgb_case *c) {
+  if (c->nxsend || c->nxrecv || c->interior_cells < FEW_CELLS) return false;
+  if (c->d_tr) return true;
+  size_t free_b = 0, total_b = 0;
+  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
+  const size_t n = (size_t)c->cells, ns = (size_t)c->phys.ns, ne = (size_t)c->ne;
+  const size_t need = sizeof(double) * n * ((c->d_state ? 0 : SW) + 2 + 2 * ns + 3 * (ne - 1) + 3 * ne);
+  return need + ((size_t)1 << 28) < free_b;
+}
+
 int prepare(pgb_case *c, bool fused) {
   if (!c->finalized) return fail(PGB_ERR_STATE, "the case is not finalized");
   RET(set_current(c));
@@ -1531,6 +1584,10 @@ int prepare(pgb_case *c, bool fused) {
     if (all != c->use_v2) c->tiles_dirty = true;
     c->use_v2 = all;
   }
+  // a grid of general metrics: the stage kernel reads 31 metric components a
+  // cell and is bound by the loads each face waits for; the passes are not
+  if (fused) c->by_passes = !c->use_v2 && passes_take(c);
+  if (fused && c->by_passes) return ensure_scratch(c);
   if (fused) {
     if (c->tiles_dirty) RET(build_tiles(c));
     RET(fused_attrs(c));
@@ -1656,7 +1713,7 @@ int pgb_case_destroy(pgb_case *c) {
     if (g) cudaGraphExecDestroy(g);
   for (auto &r : c->d_reg)
     if (r) cudaFree(r);
-  void *ptrs[] = {c->d_blks, c->d_met, c->d_dt, c->d_one, c->d_xsend, c->d_xrecv, c->d_xsvol, c->d_xrvol, c->d_halo, c->d_boxes, c->d_boxcta, c->d_boxrest, c->d_state, c->d_tr, c->d_hsp, c->d_grads,
+  void *ptrs[] = {c->d_blks, c->d_met, c->d_dt, c->d_one, c->d_xsend, c->d_xrecv, c->d_xsvol, c->d_xrvol, c->d_halo, c->d_boxes, c->d_boxcta, c->d_boxrest, c->d_boxes0, c->d_boxcta0, c->d_uref, c->d_ubad, c->d_state, c->d_tr, c->d_hsp, c->d_grads,
                   c->d_F[0], c->d_F[1], c->d_F[2], c->d_prims, c->d_tiles, c->d_counter, c->d_stage,
                   c->d_bcent, c->d_bcops, c->d_bcface[0], c->d_bcface[1], c->d_bcface[2], c->d_clock,
                   c->d_cfl, c->d_ctrl, c->d_subs, c->d_stiffhead, c->d_stiffcells, c->d_rots, c->d_nbr27};
@@ -1996,7 +2053,7 @@ int pgb_step_stage(pgb_case *c, int s, int path) {
   if (fused) {
     const auto &plan = c->plans[c->phase];
     if (s == 0) CK(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned int) * plan.size(), c->stream));
-    RET(c->form == 2 ? launch_react(c, plan[s], count) : launch_fused(c, plan[s], s, count));
+    RET(passes(c) ? launch_react(c, plan[s], count) : launch_fused(c, plan[s], s, count));
     if (s + 1 == (int)plan.size()) {
       c->phase = (c->phase + 1) % c->period;
       c->phys_of = c->maps[c->phase];
@@ -2255,6 +2312,8 @@ int pgb_case_finalize(pgb_case *c) {
   CK(cudaMalloc(&c->d_ctrl, sizeof(double) * 2));
   RET(build_bcs(c));
   CK(cudaMalloc(&c->d_counter, sizeof(unsigned int) * 16));
+  CK(cudaMalloc(&c->d_uref, sizeof(UniformRef) * c->blocks.size()));
+  CK(cudaMalloc(&c->d_ubad, sizeof(int) * c->blocks.size()));
   CK(cudaMalloc(&c->d_blks, sizeof(BlockDev) * c->blocks.size()));
   std::vector<BlockDev> devs;
   for (auto &B : c->blocks) devs.push_back(B.dev);
@@ -2286,6 +2345,21 @@ int pgb_case_finalize(pgb_case *c) {
       }
       c->nboxcta = (long long)cta.size();
       c->nboxrest = (long long)rest.size();
+    }
+    // the gradients' fill, the first layer of the faces alone, by boxes where
+    // they hold all of it
+    build_boxes(c, boxes, rest, true);
+    cells = 0;
+    for (const HaloPatch &P : boxes) cells += P.cells;
+    if (!boxes.empty() && rest.empty() && cells == c->nhalo_l0 && sim_visc(c->phys.simulator)) {
+      std::vector<int2> cta;
+      for (int q = 0; q < (int)boxes.size(); q++)
+        for (int t = 0; t < (boxes[q].cells + 255) / 256; t++) cta.push_back(make_int2(q, t));
+      CK(cudaMalloc(&c->d_boxes0, sizeof(HaloPatch) * boxes.size()));
+      CK(cudaMemcpy(c->d_boxes0, boxes.data(), sizeof(HaloPatch) * boxes.size(), cudaMemcpyHostToDevice));
+      CK(cudaMalloc(&c->d_boxcta0, sizeof(int2) * cta.size()));
+      CK(cudaMemcpy(c->d_boxcta0, cta.data(), sizeof(int2) * cta.size(), cudaMemcpyHostToDevice));
+      c->nboxcta0 = (long long)cta.size();
     }
   }
   if (!c->rots.empty()) {
@@ -2750,7 +2824,7 @@ int pgb_get_tile(const pgb_case *c, int blk, int *tw, int *th, int *kchunk) {
   if (!c || blk < 0 || blk >= (int)c->blocks.size() || !tw || !th || !kchunk) return fail(PGB_ERR_ARG, "bad argument");
   HostBlock B = c->blocks[blk];
   if (B.tw <= 0) {
-    if (c->use_v2) default_tile2(B, kV2[c->v2]);
+    if (c->use_v2) default_tile2(B, kV2[c->v2], default_ksplit(c));
     else default_tile(B);
   }
   *tw = B.tw, *th = B.th, *kchunk = B.kchunk;

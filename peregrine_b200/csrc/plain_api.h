@@ -40,8 +40,8 @@ struct PlainCase {
   long long nboxcta;
   const HaloEntry *boxrest;
   long long nboxrest;
-  // the first face layer alone as boxes (the gradients' fill), when the case
-  // lists its halo only as boxes
+  // the first face layer alone as boxes (the gradients' fill), where boxes
+  // hold all of it
   const HaloPatch *boxes0;
   const int2 *boxcta0;
   long long nboxcta0;
