@@ -189,11 +189,14 @@ __device__ inline void bc_outvelocity(const double *Qi, const double rhoinv, con
 // (the kinds' preadvflux kernels, peregrine/simulator/euler/kernels/bcs/*.mako
 // and the Navier-Stokes walls' stuckhalo and stuckhaloisot,
 // peregrine/simulator/navstokes/kernels/bcs/wall.mako:7-38)
-template <int NS, bool RG>
+// FIELDS: the velocity and, with trall, the transport and the enthalpies the
+// uniform faces read of the cell too (uniface.cuh).
+template <int NS, bool RG, bool FIELDS = false>
 __global__ void k_bc_halo(const BlockDev *__restrict__ blks, const BcFace *__restrict__ faces, int nfaces,
                           const BcEntry *__restrict__ entries, const BcOp *__restrict__ ops,
                           double *__restrict__ Qall, double *__restrict__ stall, const double *__restrict__ met,
-                          const double *__restrict__ clock, const double *__restrict__ dt, double tfrac) {
+                          const double *__restrict__ clock, const double *__restrict__ dt, double tfrac,
+                          double *__restrict__ trall = nullptr, double *__restrict__ hall = nullptr) {
   constexpr int NE = 4 + NS;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= faces[nfaces].start) return;
@@ -394,6 +397,22 @@ __global__ void k_bc_halo(const BlockDev *__restrict__ blks, const BcFace *__res
     so[4 * v] = th.e, so[5 * v] = th.cp, so[6 * v] = th.gamma, so[7 * v] = th.c;
     so[ST_Z * v] = Z;
   }
+  if (FIELDS) {
+    const State s = copy ? load_state(sb + cm, v) : th;
+    const double rhoinv = 1.0 / Qh[0];
+#pragma unroll
+    for (int m = 0; m < 3; m++) so[(ST_U + m) * v] = Qh[1 + m] * rhoinv;
+    if (trall) {
+      double tr[2 + NS], h[NS];
+      auto Qf = [&](int l) { return Qh[l]; };
+      transport<NS>(Qf, s, tr, h);
+      double *trp = trall + (2 + NS) * B.cv + ch, *hp = hall + NS * B.cv + ch;
+#pragma unroll
+      for (int n = 0; n < 2 + NS; n++) trp[n * v] = tr[n];
+#pragma unroll
+      for (int n = 0; n < NS; n++) hp[n * v] = h[n];
+    }
+  }
 }
 
 // the double flux's freeze of the boundaries' halo cells, once the halo pass
@@ -419,7 +438,7 @@ __global__ void k_bc_freeze(const BlockDev *__restrict__ blks, const BcFace *__r
 // image's (peregrine/simulator/navstokes/kernels/bcs/gradients.mako:2-6)
 template <int NS>
 __global__ void k_bc_grads(const BlockDev *__restrict__ blks, const BcFace *__restrict__ faces, int nfaces,
-                           double *__restrict__ gall) {
+                           double *__restrict__ gall, int comps) {
   constexpr int NG3 = 3 * (3 + NS);
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= faces[nfaces].start) return;
@@ -433,7 +452,8 @@ __global__ void k_bc_grads(const BlockDev *__restrict__ blks, const BcFace *__re
   double *g = gall + NG3 * B.cv;
   const long long cm = w.deep(B, layer), ch = w.halo(B, layer);
 #pragma unroll
-  for (int q = 0; q < NG3; q++) g[q * v + ch] = g[q * v + cm];
+  for (int q = 0; q < NG3; q++)
+    if (q < comps) g[q * v + ch] = g[q * v + cm];
 }
 
 // postflux of the walls: the flux through each wall face written from the

@@ -38,6 +38,7 @@ struct BlockDev {
   double xR[3];       // xf - xcc(R) along a
   // per-axis face geometry alpha damping forms, precomputed from the above
   double damp[3];     // alpha / |e . n| for an a-face (the normal is the axis)
+  int bcg;            // bit f: face f is an inflow or outflow, whose halo cells take their images' gradients
 };
 
 __host__ __device__ __forceinline__ long long cell_index(const BlockDev &b, int fi, int fj, int fk) {
@@ -59,8 +60,10 @@ __host__ __device__ __forceinline__ long long inner_cell(const BlockDev &b, long
 // realgas/model.py:31-34, realgasdf/model.py:8-10)
 constexpr int SW = 24;
 // The ideal gases leave the plane's fields unused and, on uniform blocks of the
-// fused passes, keep the cell's velocity at the record's end (uniface.cuh).
-enum { ST_Z = 8, ST_THETA = 9, ST_EPS = 10, ST_KAPPA = 11, ST_ZETA = 12, ST_U = 21 };
+// fused passes, keep the cell's velocity at the record's end (uniface.cuh); the
+// double flux's batched stages keep a second pressure there (12 species leave
+// the last field free).
+enum { ST_Z = 8, ST_THETA = 9, ST_EPS = 10, ST_KAPPA = 11, ST_ZETA = 12, ST_U = 21, ST_P2 = 23 };
 
 // Where a per-block kernel's thread works: its block and its index t in the
 // pass's range over that block.  With a tile table (a packed launch over many
@@ -95,10 +98,12 @@ __device__ __forceinline__ int face_work(const unsigned n0, const unsigned n1, c
   return axis;
 }
 // face t of an axis of a block as the index of the cell on its high side
-__device__ __forceinline__ bool face_cell(const BlockDev &B, const int axis, const unsigned t, long long &R) {
+// and its place along the axis in pos
+__device__ __forceinline__ bool face_cell(const BlockDev &B, const int axis, const unsigned t, long long &R, int &pos) {
   const unsigned fx = B.nx + (axis == 0), fy = B.ny + (axis == 1), fz = B.nz + (axis == 2);
   const unsigned r = t / fx, i = t - r * fx, k = r / fy, j = r - k * fy;
   if (k >= fz) return false;
+  pos = (int)(axis == 0 ? i : axis == 1 ? j : k);
   R = cell_index(B, (int)i + NG, (int)j + NG, (int)k + NG);
   return true;
 }

@@ -40,7 +40,7 @@ PGB_PLAIN_DECL(12)
 namespace {
 #define PGB_OPS(N)                                                                                          \
   {pgb_plain_upload_##N, pgb_plain_rhs_##N, pgb_plain_fromprims_##N, pgb_plain_production_##N, pgb_plain_prestep_##N, \
-   pgb_plain_cflmax_##N, pgb_plain_fused_##N, pgb_plain_reactors_##N, pgb_plain_reactor_prims_##N}
+   pgb_plain_cflmax_##N, pgb_plain_fused_##N, pgb_plain_bounded_##N, pgb_plain_reactors_##N, pgb_plain_reactor_prims_##N}
 // the per-block path of each species count, 1 to MAXNS
 const PlainOps kPlain[MAXNS] = {PGB_OPS(1), PGB_OPS(2), PGB_OPS(3), PGB_OPS(4),  PGB_OPS(5),  PGB_OPS(6),
                                 PGB_OPS(7), PGB_OPS(8), PGB_OPS(9), PGB_OPS(10), PGB_OPS(11), PGB_OPS(12)};
@@ -1218,13 +1218,60 @@ int cfl_prologue(pgb_case *c, int qphys, int &count) {
   return PGB_OK;
 }
 
+// a stage's combines on a register table, in place: own first, dQ as
+// src -1, the first combine's value (already in the thread) as src -2
+void stage_combines(const pgb_stage &st, double *const *reg, RCombine *out) {
+  int written0 = -1;
+  auto term = [&](RCombine &rc, int n, int r, double w) {
+    const bool dq = r < 0 || r == st.dq;
+    rc.src[n] = dq ? -1 : r == written0 ? -2 : 0;
+    rc.X[n] = rc.src[n] < 0 ? nullptr : reg[r];
+    rc.w[n] = w;
+  };
+  for (int m = 0; m < st.ncombine; m++) {
+    const pgb_combine &cb = st.combine[m];
+    RCombine &rc = out[m];
+    rc = RCombine{};
+    rc.out = reg[cb.out];
+    rc.step = cb.step;
+    rc.write = 1;
+    int n = 0;
+    if (cb.own) term(rc, n++, cb.out, cb.wout);
+    for (int q = 0; q < cb.nterms; q++) term(rc, n++, cb.reg[q], cb.w[q]);
+    rc.nterms = n;
+    if (m == 0) written0 = cb.out;
+  }
+}
+
 // whether the batched path's stages are the fused passes
 bool passes(const pgb_case *c) { return c->form == 2 || (c->form == 1 && c->by_passes); }
 
+// How a stage of the double flux comes by its state.  A face reads p alone,
+// which each stage's kernel can leave for the next, so only a step's last
+// stage forms the whole state (the next step's first guess of T, and what
+// pgb_eos_get reads); the first takes p and the halos as the step's start left
+// them.  256 x 128 x 4 cells in 8 blocks, an RK3 step 0.16 ms against 0.202 ms
+// with a state pass and a halo pass of every field each stage.  stage -1: a
+// right-hand side alone.
+void df_stage(const pgb_case *c, const FusedStagePlan &p, int stage, RStage &r) {
+  r.full = 1, r.pto = r.pm = -1;
+  if (stage < 0 || !sim_df(c->phys.simulator) || c->interior_cells < FEW_CELLS) return;
+  const auto &plan = c->plans[c->phase];
+  const int last = (int)plan.size() - 1;
+  auto field = [](int s) { return s % 2 ? ST_P2 : 0; };
+  r.full = stage == last;
+  r.pfrom = field(stage);
+  r.filled = stage == 0;
+  if (stage + 1 >= last) return;
+  for (int m = 0; m < p.ncomb; m++)
+    if (p.comb[m].out == plan[stage + 1].qin) r.pto = field(stage + 1), r.pm = m;
+}
+
 // one stage of the fused passes (react.cuh): the plan's combines on physical
 // registers; with dq set (a right-hand side alone) no combine, dQ stored there
-int launch_react(pgb_case *c, const FusedStagePlan &p, int &count, int dq = -1) {
+int launch_react(pgb_case *c, const FusedStagePlan &p, int &count, int dq = -1, int stage = -1) {
   RStage r{};
+  df_stage(c, p, stage, r);
   r.Q = c->d_reg[p.qin];
   r.dQ = c->d_reg[dq >= 0 ? dq : p.dqbuf];
   r.write_dq = dq >= 0;
@@ -1266,7 +1313,7 @@ int step_fused(pgb_case *c, int &count) {
   }
   CK(cudaMemsetAsync(c->d_counter, 0, sizeof(unsigned int) * plan.size(), c->stream));
   for (int s = 0; s < (int)plan.size(); s++)
-    RET(passes(c) ? launch_react(c, plan[s], count) : launch_fused(c, plan[s], s, count));
+    RET(passes(c) ? launch_react(c, plan[s], count, -1, s) : launch_fused(c, plan[s], s, count));
   if (c->ctrl_cfl) {
     k_clock<<<1, 1, 0, c->stream>>>(c->d_clock, c->d_dt);
     mark(c, K_COMBINE, count);
@@ -1424,7 +1471,25 @@ int df_settle(pgb_case *c, int qphys) {
   return prestep_plain(c, qphys, count, 1);
 }
 
-int rhs_plain(pgb_case *c, int qphys, int dqphys, int &count, double tfrac = 0.0) {
+// Whether a bounded case could take the uniform faces on the packed path: the
+// ideal gases' forms those take (uniform_counts), every face of every block
+// joined to a neighbour or a boundary entry, no shard.  The sub-stepped
+// chemistry keeps its passes.
+bool bounded_takes(const pgb_case *c) {
+  if (!c->nbcface[0] || c->nxsend || c->nxrecv || c->interior_cells < FEW_CELLS ||
+      c->phys.chemistry == PGB_CHEM_SUBSTEPPED)
+    return false;
+  for (const HostBlock &B : c->blocks) {
+    if (B.nx < 2 || B.ny < 2 || B.nz < 2) return false;
+    for (int f = 0; f < 6; f++)
+      if (B.nbr[f] < 0 && B.bc[f] < 0) return false;
+  }
+  return true;
+}
+
+void combine_stage(pgb_case *c, const pgb_stage &st, int &count);
+
+int rhs_plain(pgb_case *c, int qphys, int dqphys, int &count, double tfrac = 0.0, const pgb_stage *st = nullptr) {
   RET(ensure_scratch(c));
   std::vector<BlockDev> hb;
   PlainCase pc = plain_case(c, hb);
@@ -1433,6 +1498,26 @@ int rhs_plain(pgb_case *c, int qphys, int dqphys, int &count, double tfrac = 0.0
   pc.ctx = &mc;
   pc.tfrac = tfrac;
   c->state_stale = false;
+  if (c->packed && bounded_takes(c) && pc.gen == 0) {
+    // with st, the stage's combines in the same pass (dQ kept too)
+    RStage r{};
+    r.Q = c->d_reg[qphys];
+    r.dQ = c->d_reg[dqphys];
+    r.write_dq = 1;
+    pc.bcuni = 1;
+    if (st) {
+      double *reg[MAXREGS];
+      for (int q = 0; q < c->phys.nregs; q++) reg[q] = c->d_reg[c->phys_of[q]];
+      r.ncomb = st->ncombine;
+      stage_combines(*st, reg, r.comb);
+    }
+    return kPlain[c->phys.ns - 1].bounded(&pc, &r);
+  }
+  if (st) {
+    RET(kPlain[c->phys.ns - 1].rhs(&pc, c->d_reg[qphys], c->d_reg[dqphys]));
+    combine_stage(c, *st, count);
+    return PGB_OK;
+  }
   return kPlain[c->phys.ns - 1].rhs(&pc, c->d_reg[qphys], c->d_reg[dqphys]);
 }
 
@@ -1486,8 +1571,7 @@ int step_plain(pgb_case *c, int &count) {
   if (!c->stages.empty()) RET(cfl_prologue(c, map[c->stages[0].q], count));
   if (!c->stages.empty()) RET(prestep_plain(c, map[c->stages[0].q], count, 0));
   for (const pgb_stage &st : c->stages) {
-    RET(rhs_plain(c, map[st.q], map[st.dq], count, st.tfrac));
-    combine_stage(c, st, count);
+    RET(rhs_plain(c, map[st.q], map[st.dq], count, st.tfrac, &st));
   }
   // the clock moves on by dt where boundaries read it or the step size is the device's
   if (c->nbcface[0] || c->ctrl_cfl) {
@@ -1507,8 +1591,9 @@ int build_bcs(pgb_case *c) {
   long long n[3] = {0, 0, 0};
   const bool visc = sim_visc(c->phys.simulator);
   for (int b = 0; b < (int)c->blocks.size(); b++) {
-    const HostBlock &B = c->blocks[b];
+    HostBlock &B = c->blocks[b];
     const int ext[3] = {B.nx, B.ny, B.nz};
+    B.dev.bcg = 0;
     for (int f = 0; f < 6; f++) {
       const int e = B.bc[f];
       if (e < 0) continue;
@@ -1520,6 +1605,7 @@ int build_bcs(pgb_case *c) {
       if (visc && !wall) {
         t[1].push_back(BcFace{b, f, e, 0, n[1]});
         n[1] += NG * plane;
+        B.dev.bcg |= 1 << f;
       }
       if (wall) {
         t[2].push_back(BcFace{b, f, e, 0, n[2]});
@@ -1571,12 +1657,13 @@ int prepare(pgb_case *c, bool fused) {
   // the fused passes read the per-block path's state, transport, gradient
   // and face arrays, and the metric arrays of the blocks that are not uniform
   if (fused && c->form == 2) {
-    if (!c->uniform_done && !sim_df(c->phys.simulator)) RET(detect_uniform(c));
+    if (!c->uniform_done) RET(detect_uniform(c));
     return ensure_scratch(c);
   }
-  // the uniform forms are the batched path's alone: the per-block path reads
-  // the metric arrays, so a per-block call leaves the detection to the first
-  // batched step
+  // the uniform forms are the batched path's, and the packed path's for a
+  // bounded case: the per-block path reads the metric arrays, so another
+  // case's per-block call leaves the detection to the first batched step
+  if (!fused && !c->uniform_done && bounded_takes(c)) RET(detect_uniform(c));
   if (fused && !c->uniform_done) {
     RET(detect_uniform(c));
     bool all = true;
@@ -3150,30 +3237,6 @@ int pool_launch_step(pgb_pool *p, int &launches) {
   pc.ctx = &launches;
   const dim3 g((unsigned)p->nctab[R_INNER], 1, 1);
   const int2 *inner_tiles = pc.ctab[R_INNER];
-  // a stage's combines on a register table, in place: own first, dQ as
-  // src -1, the first combine's value (already in the thread) as src -2
-  auto combines = [&](const pgb_stage &st, double *const *reg, RCombine *out) {
-    int written0 = -1;
-    auto term = [&](RCombine &rc, int n, int r, double w) {
-      const bool dq = r < 0 || r == st.dq;
-      rc.src[n] = dq ? -1 : r == written0 ? -2 : 0;
-      rc.X[n] = rc.src[n] < 0 ? nullptr : reg[r];
-      rc.w[n] = w;
-    };
-    for (int m = 0; m < st.ncombine; m++) {
-      const pgb_combine &cb = st.combine[m];
-      RCombine &rc = out[m];
-      rc = RCombine{};
-      rc.out = reg[cb.out];
-      rc.step = cb.step;
-      rc.write = 1;
-      int n = 0;
-      if (cb.own) term(rc, n++, cb.out, cb.wout);
-      for (int q = 0; q < cb.nterms; q++) term(rc, n++, cb.reg[q], cb.w[q]);
-      rc.nterms = n;
-      if (m == 0) written0 = cb.out;
-    }
-  };
   for (const pgb_stage &st : p->stages) {
     if (nreac) {
       ReactorStage rs{};
@@ -3184,7 +3247,7 @@ int pool_launch_step(pgb_pool *p, int &launches) {
       rs.cap = p->rcap;
       rs.dt = p->d_dt;
       rs.ncomb = st.ncombine;
-      combines(st, p->d_rq, rs.comb);
+      stage_combines(st, p->d_rq, rs.comb);
       RET(kPlain[p->phys.ns - 1].reactors(&rs, p->stream));
       launches++;
     }
@@ -3195,7 +3258,7 @@ int pool_launch_step(pgb_pool *p, int &launches) {
       r.Q = p->d_reg[st.q];
       r.dQ = p->d_reg[st.dq];
       r.ncomb = st.ncombine;
-      combines(st, p->d_reg, r.comb);
+      stage_combines(st, p->d_reg, r.comb);
       RET(kPlain[p->phys.ns - 1].fused(&pc, &r));
       continue;
     }

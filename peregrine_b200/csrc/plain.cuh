@@ -108,11 +108,11 @@ static __global__ void __launch_bounds__(256) k_halo_boxes(double *__restrict__ 
 
 // two registers' halos in one pass over the boxes: C1 components of the
 // first (its vector at vec turned by a cell's rotation), then C2 scalar
-// components of the second; each with its own stride (0: its component
-// count).  A CTA fills 256 cells of one box, or 256 leftover entries.
+// components of the second from its component field2 on; each with its own
+// stride (0: its component count).  A CTA fills 256 cells of one box, or 256 leftover entries.
 template <int C1, int C2, bool ROT>
 static __global__ void __launch_bounds__(256) k_halo_boxes2(double *__restrict__ base1, int vec, int stride1,
-                                                            double *__restrict__ base2, int stride2,
+                                                            double *__restrict__ base2, int stride2, int field2,
                                                             const HaloPatch *__restrict__ boxes,
                                                             const int2 *__restrict__ cta,
                                                             const HaloEntry *__restrict__ rest, long long nrest,
@@ -125,7 +125,8 @@ static __global__ void __launch_bounds__(256) k_halo_boxes2(double *__restrict__
     if (t >= nrest) return;
     const HaloEntry h = rest[t];
     halo_copy<C1, ROT>(base1, C1, vec, rots, h.dcv, h.didx, h.dvol, h.scv, h.sidx, h.svol, h.rot, stride1);
-    halo_copy<C2, false>(base2, C2, HALO_SCALARS, rots, h.dcv, h.didx, h.dvol, h.scv, h.sidx, h.svol, 0, stride2);
+    halo_copy<C2, false>(base2, C2, HALO_SCALARS, rots, h.dcv, h.didx + (long long)field2 * h.dvol, h.dvol, h.scv,
+                         h.sidx + (long long)field2 * h.svol, h.svol, 0, stride2);
     return;
   }
   const HaloPatch &p = boxes[w.x];
@@ -134,7 +135,8 @@ static __global__ void __launch_bounds__(256) k_halo_boxes2(double *__restrict__
   const int didx = p.d0 + x0 * p.dst[0] + x1 * p.dst[1] + x2 * p.dst[2];
   const int sidx = p.s0 + x0 * p.sst[0] + x1 * p.sst[1] + x2 * p.sst[2];
   halo_copy<C1, ROT>(base1, C1, vec, rots, p.dcv, didx, p.dvol, p.scv, sidx, p.svol, p.rot, stride1);
-  halo_copy<C2, false>(base2, C2, HALO_SCALARS, rots, p.dcv, didx, p.dvol, p.scv, sidx, p.svol, 0, stride2);
+  halo_copy<C2, false>(base2, C2, HALO_SCALARS, rots, p.dcv, didx + (long long)field2 * p.dvol, p.dvol, p.scv,
+                       sidx + (long long)field2 * p.svol, p.svol, 0, stride2);
 }
 
 // the box fill of a register of comps components: the kernel built for that

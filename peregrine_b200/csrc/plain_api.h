@@ -84,6 +84,7 @@ struct PlainCase {
   // cell's filled from its source's in one pass (a shard's traded halo cells
   // get Q alone, so its fields are formed in place)
   int uni, gen, fill_all;
+  int bcuni;  // a bounded case, packed, whose stages are pgb_plain_bounded's
   int few;  // a case of few cells: the faces a launch an axis
   int tpg;  // thermally perfect (else calorically)
   double tfrac;
@@ -110,6 +111,11 @@ struct RStage {
   int write_dq;
   int ncomb;
   RCombine comb[2];
+  // the double flux: whether this stage forms the whole state (a step's last,
+  // and a right-hand side alone), else the field its faces read p from and
+  // whether its halo was filled with the planes'; and the field the next
+  // stage's p goes to (-1: none), off combine pm's Q
+  int full, pfrom, filled, pto, pm;
 };
 
 // the serving pool's reactors' stage (react.cuh, k_reactors): the stage's
@@ -134,6 +140,7 @@ struct PlainOps {
   int (*prestep)(const PlainCase *, double *Q, int first);
   int (*cflmax)(const PlainCase *, const double *Q, double *out);
   int (*fused)(const PlainCase *, const RStage *);
+  int (*bounded)(const PlainCase *, const RStage *);
   int (*reactors)(const ReactorStage *, cudaStream_t);
   int (*reactor_prims)(const double *prims, double *Q, double *T, int row, long long cap, cudaStream_t);
 };
@@ -155,6 +162,8 @@ struct PlainOps {
                                                                             double *);                           \
   extern "C" __attribute__((visibility("hidden"))) int pgb_plain_fused_##N(const pgb::PlainCase *,               \
                                                                            const pgb::RStage *);                 \
+  extern "C" __attribute__((visibility("hidden"))) int pgb_plain_bounded_##N(const pgb::PlainCase *,             \
+                                                                             const pgb::RStage *);               \
   extern "C" __attribute__((visibility("hidden"))) int pgb_plain_reactors_##N(const pgb::ReactorStage *,         \
                                                                               cudaStream_t);                     \
   extern "C" __attribute__((visibility("hidden"))) int pgb_plain_reactor_prims_##N(                              \

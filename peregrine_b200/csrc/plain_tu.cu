@@ -239,8 +239,15 @@ extern "C" int PGB_ENTRY(pgb_plain_upload_)(const Species *sp, const Mech *mech,
 // gradients (after the gradients' exchange) and the walls' face fluxes (after
 // the flux functions, before the divergence), one launch each over every
 // block's boundary faces
-static void bc_halo_launch(const PlainCase *pc, const double *Q) {
+static void bc_halo_launch(const PlainCase *pc, const double *Q, const bool fields = false) {
   if (!pc->nbchalo) return;
+  if (fields) {
+    k_bc_halo<NS, false, true><<<grid_of(pc->bchalo_n), TH, 0, pc->stream>>>(
+        pc->d_blks, pc->bchalo, pc->nbchalo, pc->bcent, pc->bcops, const_cast<double *>(Q), pc->state, pc->met,
+        pc->clock, pc->dt, pc->tfrac, pc->visc ? pc->tr : nullptr, pc->hsp);
+    mark(pc, 4);
+    return;
+  }
   if (pc->realgas)
     k_bc_halo<NS, true><<<grid_of(pc->bchalo_n), TH, 0, pc->stream>>>(
         pc->d_blks, pc->bchalo, pc->nbchalo, pc->bcent, pc->bcops, const_cast<double *>(Q), pc->state, pc->met,
@@ -251,9 +258,9 @@ static void bc_halo_launch(const PlainCase *pc, const double *Q) {
         pc->clock, pc->dt, pc->tfrac);
   mark(pc, 4);
 }
-static void bc_grads_launch(const PlainCase *pc) {
+static void bc_grads_launch(const PlainCase *pc, const int comps = 3 * (NE - 1)) {
   if (!pc->nbcgrad) return;
-  k_bc_grads<NS><<<grid_of(pc->bcgrad_n), TH, 0, pc->stream>>>(pc->d_blks, pc->bcgrad, pc->nbcgrad, pc->grads);
+  k_bc_grads<NS><<<grid_of(pc->bcgrad_n), TH, 0, pc->stream>>>(pc->d_blks, pc->bcgrad, pc->nbcgrad, pc->grads, comps);
   mark(pc, 4);
 }
 static void bc_wall_launch(const PlainCase *pc, const double *Q) {
@@ -463,10 +470,10 @@ extern "C" int PGB_ENTRY(pgb_plain_prestep_)(const PlainCase *pc, double *Q, int
   if (pc->boxcta && pc->nboxcta > 0) {
     // Q's halo and the state's (planes included) in one pass over the boxes
     if (pc->rots)
-      k_halo_boxes2<NE, CS, true><<<(unsigned)pc->nboxcta, 256, 0, s>>>(Q, 1, 0, pc->state, SW, pc->boxes, pc->boxcta,
+      k_halo_boxes2<NE, CS, true><<<(unsigned)pc->nboxcta, 256, 0, s>>>(Q, 1, 0, pc->state, SW, 0, pc->boxes, pc->boxcta,
                                                                         pc->boxrest, pc->nboxrest, pc->rots);
     else
-      k_halo_boxes2<NE, CS, false><<<(unsigned)pc->nboxcta, 256, 0, s>>>(Q, 1, 0, pc->state, SW, pc->boxes, pc->boxcta,
+      k_halo_boxes2<NE, CS, false><<<(unsigned)pc->nboxcta, 256, 0, s>>>(Q, 1, 0, pc->state, SW, 0, pc->boxes, pc->boxcta,
                                                                          pc->boxrest, pc->nboxrest, pc->rots);
     mark(pc, 0);
   } else {
@@ -508,6 +515,9 @@ void rgrads_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const voi
   const RStage &r = *(const RStage *)ctx;
   k_grads<NS><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->met, pc->grads, 0, ct);
 }
+void vgrads_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *) {
+  k_vgrads<NS><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, pc->state, pc->grads, ct);
+}
 // the CTAs a block takes of each axis of a pass over every face, and the grid's
 // rows; with tile tables (which lie axis after axis) two CTAs a tile
 bool face_grid(const PlainCase *pc, unsigned *n, unsigned &rows) {
@@ -529,7 +539,8 @@ void ufaces_go(const PlainCase *pc, const RStage *r, int lim) {
   unsigned n[3], rows;
   if (!face_grid(pc, n, rows)) return;
   k_ufaces<NS, FN, KOREN, VISC, TPG><<<dim3(n[0] + n[1] + n[2], rows, 1), UF_TH, 0, pc->stream>>>(
-      pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->F[0], pc->F[1], pc->F[2], lim, n[0], n[1], pc->ctab[R_FX]);
+      pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->bcuni ? pc->grads : nullptr, pc->F[0], pc->F[1], pc->F[2], lim,
+      n[0], n[1], pc->ctab[R_FX]);
   mark(pc, 2);
 }
 template <bool VISC, bool TPG>
@@ -581,15 +592,54 @@ void rapply_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const voi
   const RApplyCtx &r = *(const RApplyCtx *)ctx;
   k_rapply<NS><<<dim3(g.x, g.y, NE), TH, 0, pc->stream>>>(pc->d_blks, b, pc->F[0], pc->F[1], pc->F[2], pc->met, r.a, ct);
 }
-struct RCellFluxCtx {
-  const double *Q;
-  RApplyArgs a;
-};
-void rcellflux_df_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
-  const RCellFluxCtx &r = *(const RCellFluxCtx *)ctx;
-  k_rcellflux_df<NS><<<g, TH, 0, pc->stream>>>(pc->d_blks, b, r.Q, pc->state, pc->met, r.a, ct);
+void rcellflux_df_launch(const PlainCase *pc, const RStage *r, const RApplyArgs &a, int pfrom, int pto) {
+  constexpr int T = 128;
+  long long most = 0;
+  for (int b = 0; b < pc->nblocks; b++) most = std::max(most, range_size(pc->h_blks[b], R_INNER));
+  if (pc->nblocks > 0)
+    k_rcellflux_df<NS><<<dim3((unsigned)((most + T - 1) / T), (unsigned)pc->nblocks, 1), T, 0, pc->stream>>>(
+        pc->d_blks, 0, r->Q, pc->state, pc->met, a, pfrom, pto, r->pm);
+  mark(pc, 1);
 }
 }  // namespace
+
+// One stage of a bounded case on uniform blocks, packed: the fused passes'
+// kernels with the boundaries' passes between them.  The velocity's gradients
+// go by arrays here, as a boundary's halo cells take their images'
+extern "C" int PGB_ENTRY(pgb_plain_bounded_)(const PlainCase *pc, const RStage *rs) {
+  halo_fill(pc, const_cast<double *>(rs->Q), NE, 1);
+  mark(pc, 0);
+  for_blocks(pc, R_VOL, pc->visc ? rcell_launch<true> : rcell_launch<false>, rs, 2);
+  bc_halo_launch(pc, rs->Q, true);
+  if (pc->visc) {
+    for_blocks(pc, R_INNER, vgrads_launch, rs, 2);
+    constexpr int NG3 = 3 * (NE - 1);
+    if (pc->boxcta0 && pc->nboxcta0 > 0)
+      halo_boxes_launch<9>((unsigned)pc->nboxcta0, pc->stream, pc->grads, pc->boxes0, pc->boxcta0, nullptr, 0, 9,
+                           HALO_TENSOR, pc->rots, NG3);
+    else
+      k_halo<<<grid_of(pc->nhalo_l0), TH, 0, pc->stream>>>(pc->grads, pc->halo, pc->nhalo_l0, 9, HALO_TENSOR, pc->rots,
+                                                          NG3);
+    mark(pc, 0);
+    bc_grads_launch(pc, 9);
+  }
+  const bool chem = pc->chem == PGB_CHEM_COUPLED;
+  if (chem) for_blocks(pc, R_INNER, rsource_launch, rs, 2);
+  if (pc->tpg) pc->visc ? ufaces_launch<true, true>(pc, rs) : ufaces_launch<false, true>(pc, rs);
+  else pc->visc ? ufaces_launch<true, false>(pc, rs) : ufaces_launch<false, false>(pc, rs);
+  bc_wall_launch(pc, rs->Q);
+  RApplyCtx ra{};
+  ra.a.dQ = rs->dQ;
+  ra.a.dt = pc->dt;
+  ra.a.chem = chem ? 1 : 0;
+  ra.a.write_dq = rs->write_dq;
+  ra.a.ncomb = rs->ncomb;
+  ra.a.comb[0] = rs->comb[0];
+  ra.a.comb[1] = rs->comb[1];
+  for_blocks(pc, R_INNER, rapply_launch, &ra, 2);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? PGB_OK : cuda_fail(e, "bounded stage");
+}
 
 extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs) {
   cudaStream_t s = pc->stream;
@@ -599,7 +649,10 @@ extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs
   // the other gases likewise: the interior's fields, then Q's halo and every
   // field's in one pass over the boxes
   const bool inner = !pc->df && pc->fill_all && pc->boxcta && pc->nboxcta > 0;
-  if (!df_inner && !inner) {
+  // a stage of the double flux that is not the whole state's takes p off the
+  // field the stage before (or the step's start) left it in
+  const bool chain = pc->df && pc->boxcta && pc->nboxcta > 0, light = chain && !rs->full;
+  if (!light && !df_inner && !inner) {
     halo_fill(pc, const_cast<double *>(rs->Q), NE, 1);
     mark(pc, 0);
   }
@@ -608,7 +661,20 @@ extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs
     // plane (halo included), then a cell a thread of its six faces, the
     // divergence and the combines
     const RhsArgs q{rs->Q, rs->dQ};
-    if (df_inner) {
+    if (light) {
+      // Q's halo and p's, unless the step's start has just filled both
+      if (!rs->filled) {
+        if (pc->rots)
+          k_halo_boxes2<NE, 1, true><<<(unsigned)pc->nboxcta, 256, 0, s>>>(
+              const_cast<double *>(rs->Q), 1, 0, pc->state, SW, rs->pfrom, pc->boxes, pc->boxcta, pc->boxrest,
+              pc->nboxrest, pc->rots);
+        else
+          k_halo_boxes2<NE, 1, false><<<(unsigned)pc->nboxcta, 256, 0, s>>>(
+              const_cast<double *>(rs->Q), 1, 0, pc->state, SW, rs->pfrom, pc->boxes, pc->boxcta, pc->boxrest,
+              pc->nboxrest, pc->rots);
+        mark(pc, 0);
+      }
+    } else if (df_inner) {
       // the interior's state, then in one pass over the halo Q's halo and
       // each halo cell's state (p .. c and Z) copied from its source's: the
       // values the pass would form there, as a halo cell's Q, frozen plane
@@ -617,24 +683,22 @@ extern "C" int PGB_ENTRY(pgb_plain_fused_)(const PlainCase *pc, const RStage *rs
       constexpr int CS = ST_Z + 1;
       if (pc->rots)
         k_halo_boxes2<NE, CS, true><<<(unsigned)pc->nboxcta, 256, 0, s>>>(
-            const_cast<double *>(rs->Q), 1, 0, pc->state, SW, pc->boxes, pc->boxcta, pc->boxrest, pc->nboxrest, pc->rots);
+            const_cast<double *>(rs->Q), 1, 0, pc->state, SW, 0, pc->boxes, pc->boxcta, pc->boxrest, pc->nboxrest, pc->rots);
       else
         k_halo_boxes2<NE, CS, false><<<(unsigned)pc->nboxcta, 256, 0, s>>>(
-            const_cast<double *>(rs->Q), 1, 0, pc->state, SW, pc->boxes, pc->boxcta, pc->boxrest, pc->nboxrest, pc->rots);
+            const_cast<double *>(rs->Q), 1, 0, pc->state, SW, 0, pc->boxes, pc->boxcta, pc->boxrest, pc->nboxrest, pc->rots);
       mark(pc, 0);
     } else {
       for_blocks(pc, R_VOL, fromQ_launch, &q, 8);
     }
-    RCellFluxCtx cf{};
-    cf.Q = rs->Q;
-    RApplyArgs &a = cf.a;
+    RApplyArgs a{};
     a.dQ = rs->dQ;
     a.dt = pc->dt;
     a.write_dq = rs->write_dq;
     a.ncomb = rs->ncomb;
     a.comb[0] = rs->comb[0];
     a.comb[1] = rs->comb[1];
-    for_blocks(pc, R_INNER, rcellflux_df_launch, &cf, 1);
+    rcellflux_df_launch(pc, rs, a, light ? rs->pfrom : 0, light ? rs->pto : -1);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PGB_OK : cuda_fail(e, "fused double-flux stage");
   }

@@ -137,7 +137,8 @@ __global__ void __launch_bounds__(RF_TH, 4) k_rface(const BlockDev *__restrict__
   // the uniform blocks' faces are k_ufaces'
   if (skipu && B.uniform) return;
   long long R;
-  if (!face_cell(B, axis, t, R)) return;
+  int pos;
+  if (!face_cell(B, axis, t, R, pos)) return;
   double F[NE];
   const double *Q = Qall + NE * B.cv, *st = stall + SW * B.cv, *M = met + M_NCOMP * B.cv;
   const double *tr = VISC ? trall + (2 + NS) * B.cv : nullptr, *hs = VISC ? hall + NS * B.cv : nullptr;
@@ -196,6 +197,60 @@ __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blk
   }
 }
 
+// What a double-flux face reads of a cell: velocity, pressure, density and its
+// reciprocal, the carried mass fractions and the frozen plane
+template <int NS>
+struct DFCell {
+  double u, v, w, p, rho, ri, th, ep, ka;
+  double Y[NS > 1 ? NS - 1 : 1], ze[NS > 1 ? NS - 1 : 1];
+};
+
+// the cell at c (an index into the block's arrays Q and st, component stride
+// v), its pressure in the state's field pf
+template <int NS>
+__device__ __forceinline__ DFCell<NS> df_cell(const double *__restrict__ Q, const double *__restrict__ st,
+                                              const long long v, const long long c, const int pf) {
+  DFCell<NS> x;
+  const double q0 = Q[c], q1 = Q[v + c], q2 = Q[2 * v + c], q3 = Q[3 * v + c];
+  x.p = st[pf * v + c];
+  x.th = st[ST_THETA * v + c], x.ep = st[ST_EPS * v + c], x.ka = st[ST_KAPPA * v + c];
+#pragma unroll
+  for (int n = 0; n < NS - 1; n++) x.Y[n] = Q[(5 + n) * v + c], x.ze[n] = st[(ST_ZETA + n) * v + c];
+  x.rho = q0;
+  x.ri = 1.0 / q0;
+  x.u = q1 * x.ri, x.v = q2 * x.ri, x.w = q3 * x.ri;
+#pragma unroll
+  for (int n = 0; n < NS - 1; n++) x.Y[n] *= x.ri;
+  return x;
+}
+
+// the double flux's kepaec of the face between L and R (advflux_df_face,
+// plain.cuh), the energy row in R's frozen plane with RPLANE, else in L's
+template <int NS, bool RPLANE>
+__device__ __forceinline__ void df_face(const DFCell<NS> &L, const DFCell<NS> &R, const double S0, const double S1,
+                                        const double S2, double *F) {
+  const double uf = 0.5 * (R.u + L.u), vf = 0.5 * (R.v + L.v), wf = 0.5 * (R.w + L.w);
+  const double U = S0 * uf + S1 * vf + S2 * wf;
+  const double pf = 0.5 * (R.p + L.p);
+  const double C = 0.5 * (R.rho + L.rho) * U;
+  F[0] = C;
+  F[1] = C * uf + pf * S0;
+  F[2] = C * vf + pf * S1;
+  F[3] = C * wf + pf * S2;
+  const double Kj = C * 0.5 * (R.u * L.u + R.v * L.v + R.w * L.w);
+  const double Pj = 0.5 * (L.p * (R.u * S0 + R.v * S1 + R.w * S2) + R.p * (L.u * S0 + L.v * S1 + L.w * S2));
+  const DFCell<NS> &P = RPLANE ? R : L;
+  double comp = 0.0;
+#pragma unroll
+  for (int n = 0; n < NS - 1; n++) {
+    const double Ys = R.Y[n] + L.Y[n];
+    F[5 + n] = 0.5 * Ys * C;
+    comp += P.ze[n] * Ys;
+  }
+  const double tL = (P.th * L.p + P.ka) * L.ri, tR = (P.th * R.p + P.ka) * R.ri;
+  F[4] = (P.ep + 0.5 * comp + 2.0 * tL * tR / (tL + tR)) * C + Kj + Pj;
+}
+
 // The double flux's stage for an inviscid gas with kepaec, a cell a thread:
 // its six faces' two-point fluxes (each face formed by both cells it joins;
 // kepaec reads the two cells alone), the divergence in the per-block
@@ -203,64 +258,57 @@ __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blk
 // cell's low faces, where it is the right cell, the first on its high
 // faces), and the stage's combines
 // (peregrine/simulator/eulerdf/kernels/flux/function/kepaec.mako:1-21,
-//  peregrine/simulator/eulerdf/kernels/applyflux.mako:2-14)
+//  peregrine/simulator/eulerdf/kernels/applyflux.mako:2-14).
+//
+// The cell is read once and kept for its six faces, a neighbour's velocity is
+// its momentum times one reciprocal, and a face's energy is formed in this
+// cell's plane alone: 7 cells' loads and 19 divisions where each face reading
+// its two cells took 12 and 72.  A face reads no thermodynamics but p (field
+// pf of the state), which comes off the frozen plane, so with pto >= 0 the
+// cell's p for the next stage is formed here from combine pm's new Q, into
+// field pto: that stage then needs no state pass.
 template <int NS>
-__global__ void __launch_bounds__(256) k_rcellflux_df(const BlockDev *__restrict__ blks, int b,
-                                                      const double *__restrict__ Qall,
-                                                      const double *__restrict__ stall,
+__global__ void __launch_bounds__(128) k_rcellflux_df(const BlockDev *__restrict__ blks, int b,
+                                                      const double *__restrict__ Qall, double *__restrict__ stall,
                                                       const double *__restrict__ met, const RApplyArgs a,
-                                                      const int2 *__restrict__ ctab = nullptr) {
-  constexpr int NE = 4 + NS, NF = NE + 1;
-  PGB_WHERE(B, t);
+                                                      const int pf, const int pto, const int pm) {
+  constexpr int NE = 4 + NS;
+  const BlockDev &B = blks[b + (int)blockIdx.y];
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= (long long)B.nx * B.ny * B.nz) return;
-  const int i = (int)(t % B.nx) + NG, j = (int)((t / B.nx) % B.ny) + NG, k = (int)(t / ((long long)B.nx * B.ny)) + NG;
-  const long long c = cell_index(B, i, j, k), v = B.vol;
-  const long long sJ = B.X, sK = (long long)B.X * B.Y;
-  const double *Q = Qall + NE * B.cv, *st = stall + SW * B.cv, *M = met + M_NCOMP * B.cv;
-  // the six faces one after another, each summed in as it is formed, in
-  // the divergence's order (low i, j, k faces added, high ones taken off):
-  // one face's rows live at a time
+  const long long c = inner_cell(B, t), v = B.vol;
+  const double *Q = Qall + NE * B.cv, *M = met + M_NCOMP * B.cv;
+  double *st = stall + SW * B.cv;
+  const DFCell<NS> me = df_cell<NS>(Q, st, v, c, pf);
+  // the faces one after another, each summed in as it is formed, in the
+  // divergence's order (low i, j, k faces added, high ones taken off)
   double acc[NE];
-  {
-    double f[NF];
-    advflux_df_face<NS, 0>(B, Q, st, M, c, f);
 #pragma unroll
-    for (int l = 0; l < NE; l++) acc[l] = f[l == 4 ? NE : l];
-  }
-  {
-    double f[NF];
-    advflux_df_face<NS, 1>(B, Q, st, M, c, f);
+  for (int l = 0; l < NE; l++) acc[l] = 0.0;
 #pragma unroll
-    for (int l = 0; l < NE; l++) acc[l] = acc[l] + f[l == 4 ? NE : l];
-  }
-  {
-    double f[NF];
-    advflux_df_face<NS, 2>(B, Q, st, M, c, f);
+  for (int f = 0; f < 6; f++) {
+    const int A = f % 3;
+    const bool low = f < 3;
+    const long long d = A == 0 ? 1 : A == 1 ? B.X : (long long)B.X * B.Y;
+    const long long at = low ? c : c + d;
+    double S[3] = {0.0, 0.0, 0.0};
+    if (B.uniform) {
+      S[A] = B.S[A];
+    } else {
 #pragma unroll
-    for (int l = 0; l < NE; l++) acc[l] = acc[l] + f[l == 4 ? NE : l];
-  }
-  {
-    double f[NF];
-    advflux_df_face<NS, 0>(B, Q, st, M, c + 1, f);
+      for (int e = 0; e < 3; e++) S[e] = M[(M_S + 3 * A + e) * v + at];
+    }
+    const DFCell<NS> nb = df_cell<NS>(Q, st, v, low ? c - d : c + d, pf);
+    double F[NE];
+    if (low) df_face<NS, true>(nb, me, S[0], S[1], S[2], F);
+    else df_face<NS, false>(me, nb, S[0], S[1], S[2], F);
 #pragma unroll
-    for (int l = 0; l < NE; l++) acc[l] = acc[l] - f[l];
+    for (int l = 0; l < NE; l++) acc[l] = f == 0 ? F[l] : low ? acc[l] + F[l] : acc[l] - F[l];
   }
-  {
-    double f[NF];
-    advflux_df_face<NS, 1>(B, Q, st, M, c + sJ, f);
-#pragma unroll
-    for (int l = 0; l < NE; l++) acc[l] = acc[l] - f[l];
-  }
-  {
-    double f[NF];
-    advflux_df_face<NS, 2>(B, Q, st, M, c + sK, f);
-#pragma unroll
-    for (int l = 0; l < NE; l++) acc[l] = acc[l] - f[l];
-  }
-  const double detJinv = M[M_DETJINV * v + c];
+  const double detJinv = B.uniform ? B.detJinv : M[M_DETJINV * v + c];
   const long long at = NE * B.cv + c;
   const double dt = *a.dt;
-  double first[NE];
+  double first[NE], qn[NE];
 #pragma unroll
   for (int l = 0; l < NE; l++) {
     const double dq = div_begin(acc[l], detJinv);
@@ -275,8 +323,17 @@ __global__ void __launch_bounds__(256) k_rcellflux_df(const BlockDev *__restrict
       double acc = term_first(weight(0), val(0));
       for (int n = 1; n < cb.nterms; n++) acc = term_next(acc, weight(n), val(n));
       if (m == 0) first[l] = acc;
+      if (m == pm) qn[l] = acc;
       if (cb.write) cb.out[at + l * v] = acc;
     }
+  }
+  if (pto >= 0) {
+    // pplane (peregrine/simulator/mixture/eos/realgasdf/kernels/eos.mako:50-56)
+    double comp = 0.0;
+#pragma unroll
+    for (int n = 0; n < NS - 1; n++) comp += me.ze[n] * qn[5 + n];
+    st[pto * v + c] = (qn[4] - 0.5 * (qn[1] * qn[1] + qn[2] * qn[2] + qn[3] * qn[3]) / qn[0] - me.ep * qn[0] - comp -
+                       me.ka) / me.th;
   }
 }
 

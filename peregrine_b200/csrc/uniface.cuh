@@ -130,11 +130,14 @@ __device__ __forceinline__ void riemann_axis(const RSide &L, const RSide &R, con
 // the face of axis A of a uniform block whose high-side cell is R into
 // F[NE]; FN 0 is kepaec on the cells as they are, else a Riemann solver on
 // MUSCL's sides under limiter lim.  Q, st, tr, hs the block's own arrays;
-// st's fields ST_U.. hold the cells' velocities.
+// st's fields ST_U.. hold the cells' velocities.  gr, when given, holds the
+// cells' velocity gradients (a bounded block's: its halo cells' are set by the
+// boundaries); lo, hi: the low or high cell is a boundary's halo cell whose
+// gradient is the other's.
 template <int NS, int A, int FN, bool KOREN, bool VISC, bool TPG>
 __device__ __forceinline__ void uface(const BlockDev &B, const double *__restrict__ Q, const double *__restrict__ st,
-                                      const double *__restrict__ tr, const double *__restrict__ hs, const int limiter,
-                                      const long long R, double *__restrict__ Fo, double *sh) {
+                                      const double *__restrict__ tr, const double *__restrict__ hs, const double *__restrict__ gr,
+                                      const bool lo, const bool hi, const int limiter, const long long R, double *__restrict__ Fo, double *sh) {
   const int lim = KOREN ? LIM_KOREN : limiter;
   constexpr int B1 = (A + 1) % 3, B2 = (A + 2) % 3;
   const int step[3] = {1, B.X, B.X * B.Y};
@@ -149,7 +152,7 @@ __device__ __forceinline__ void uface(const BlockDev &B, const double *__restric
   // the jump the sides' extrapolations leave at the face
   const double damp = VISC ? B.damp[A] : 0.0, xL = B.xL[A], xR = B.xR[A];
   auto along = [&](const double LL, const double L, const double Rr, const double RR) {
-    const double gL = hJ * (Rr - LL), gR = hJ * (RR - L);
+    const double dL = hJ * (Rr - LL), dR = hJ * (RR - L), gL = lo ? dR : dL, gR = hi ? dL : dR;
     return 0.5 * (gR + gL) + damp * ((Rr + gR * xR) - (L + gL * xL));
   };
   if (VISC) {
@@ -169,6 +172,7 @@ __device__ __forceinline__ void uface(const BlockDev &B, const double *__restric
     }
     // across A: the mean of the two cells' central differences
     auto across = [&](const int m, const int b) {
+      if (gr) return 0.5 * (gr[(3 * m + b) * v + R] + gr[(3 * m + b) * v + R - d]);
       const double *u = st + (ST_U + m) * v;
       const int s = step[b];
       const double gL = u[s - d] - u[-s - d], gR = u[s] - u[-s];
@@ -286,11 +290,31 @@ __device__ __forceinline__ void uface(const BlockDev &B, const double *__restric
   }
 }
 
+// the velocity's gradients on the interior of the uniform blocks, rows u, v, w
+// of the gradient arrays, from the velocity the cell pass keeps
+template <int NS>
+__global__ void __launch_bounds__(256) k_vgrads(const BlockDev *__restrict__ blks, int b,
+                                                const double *__restrict__ stall, double *__restrict__ gall,
+                                                const int2 *__restrict__ ctab = nullptr) {
+  PGB_WHERE(B, t);
+  if (t >= (long long)B.nx * B.ny * B.nz) return;
+  const long long c = inner_cell(B, t), v = B.vol;
+  const double *st = stall + SW * B.cv + ST_U * v + c;
+  double *g = gall + 3 * (3 + NS) * B.cv + c;
+  const int step[3] = {1, B.X, B.X * B.Y};
+#pragma unroll
+  for (int m = 0; m < 3; m++)
+#pragma unroll
+    for (int e = 0; e < 3; e++)
+      g[(3 * m + e) * v] = 0.5 * (st[m * v + step[e]] - st[m * v - step[e]]) * B.Jd[e];
+}
+
 // the faces of every uniform block, all three axes in one launch
 template <int NS, int FN, bool KOREN, bool VISC, bool TPG>
 __global__ void __launch_bounds__(UF_TH, TPG ? 4 : 5) k_ufaces(const BlockDev *__restrict__ blks, const double *__restrict__ Qall,
                                                      const double *__restrict__ stall, const double *__restrict__ trall,
-                                                     const double *__restrict__ hall, double *F0, double *F1,
+                                                     const double *__restrict__ hall,
+                                                     const double *__restrict__ gall, double *F0, double *F1,
                                                      double *F2, const int lim, const unsigned n0, const unsigned n1,
                                                      const int2 *__restrict__ ctab) {
   constexpr int NE = 4 + NS;
@@ -300,15 +324,19 @@ __global__ void __launch_bounds__(UF_TH, TPG ? 4 : 5) k_ufaces(const BlockDev *_
   const BlockDev &B = blks[row];
   if (!B.uniform) return;
   long long R;
-  if (!face_cell(B, axis, t, R)) return;
+  int pos;
+  if (!face_cell(B, axis, t, R, pos)) return;
+  const bool lo = pos == 0 && (B.bcg >> (2 * axis) & 1);
+  const bool hi = pos == (axis == 0 ? B.nx : axis == 1 ? B.ny : B.nz) && (B.bcg >> (2 * axis + 1) & 1);
+  const double *gr = VISC && gall ? gall + 3 * (NE - 1) * B.cv : nullptr;
   const double *Q = Qall + NE * B.cv, *st = stall + SW * B.cv;
   const double *tr = VISC ? trall + (2 + NS) * B.cv : nullptr, *hs = VISC ? hall + NS * B.cv : nullptr;
   const long long at = NE * B.cv;
   __shared__ double flux[VISC ? (NS > 1 ? NS - 1 : 1) * UF_TH : 1];
   double *sh = flux + (VISC ? threadIdx.x : 0);
-  if (axis == 0) uface<NS, 0, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, lim, R, F0 + at, sh);
-  else if (axis == 1) uface<NS, 1, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, lim, R, F1 + at, sh);
-  else uface<NS, 2, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, lim, R, F2 + at, sh);
+  if (axis == 0) uface<NS, 0, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, lo, hi, lim, R, F0 + at, sh);
+  else if (axis == 1) uface<NS, 1, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, lo, hi, lim, R, F1 + at, sh);
+  else uface<NS, 2, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, lo, hi, lim, R, F2 + at, sh);
 }
 
 // every field the faces read of a halo cell, in one pass over the halo's
