@@ -567,20 +567,26 @@ void rface_launch(const PlainCase *pc, const RStage *r, const int only = -1) {
     if (only >= 0 && a != only) n[a] = 0;
   const dim3 g(n[0] + n[1] + n[2], rows, 1);
   cudaStream_t s = pc->stream;
-#define PGB_RFACE(FN)                                                                                             \
+#define PGB_RFACE(FN, K)                                                                                           \
   if (pc->visc)                                                                                                 \
-    k_rface<NS, FN, true><<<g, RF_TH, 0, s>>>(pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->grads, pc->met, \
+    k_rface<NS, FN, K, true><<<g, RF_TH, 0, s>>>(pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->grads, pc->met, \
                                               pc->F[0], pc->F[1], pc->F[2], lim, pc->uni > 0, n[0], n[1],       \
                                               pc->ctab[R_FX]);                                                  \
   else                                                                                                          \
-    k_rface<NS, FN, false><<<g, RF_TH, 0, s>>>(pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->grads, pc->met, \
+    k_rface<NS, FN, K, false><<<g, RF_TH, 0, s>>>(pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->grads, pc->met, \
                                                pc->F[0], pc->F[1], pc->F[2], lim, pc->uni > 0, n[0], n[1],      \
                                                pc->ctab[R_FX]);
   switch (pc->primary) {
-    case PGB_FLUX_KEPAEC: PGB_RFACE(0) break;
-    case PGB_FLUX_HLLC: PGB_RFACE(FN_HLLC) break;
-    case PGB_FLUX_RUSANOV: PGB_RFACE(FN_RUSANOV) break;
-    default: PGB_RFACE(FN_AUSMUP) break;
+    case PGB_FLUX_KEPAEC: PGB_RFACE(0, false) break;
+    case PGB_FLUX_HLLC:
+      if (lim == LIM_KOREN) {
+        PGB_RFACE(FN_HLLC, true)
+      } else {
+        PGB_RFACE(FN_HLLC, false)
+      }
+      break;
+    case PGB_FLUX_RUSANOV: PGB_RFACE(FN_RUSANOV, false) break;
+    default: PGB_RFACE(FN_AUSMUP, false) break;
   }
 #undef PGB_RFACE
   mark(pc, 2);
@@ -590,7 +596,7 @@ struct RApplyCtx {
 };
 void rapply_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
   const RApplyCtx &r = *(const RApplyCtx *)ctx;
-  k_rapply<NS><<<dim3(g.x, g.y, NE), TH, 0, pc->stream>>>(pc->d_blks, b, pc->F[0], pc->F[1], pc->F[2], pc->met, r.a, ct);
+  k_rapply<NS><<<dim3(g.x, g.y, (NE + RA_COMPS - 1) / RA_COMPS), TH, 0, pc->stream>>>(pc->d_blks, b, pc->F[0], pc->F[1], pc->F[2], pc->met, r.a, ct);
 }
 void rcellflux_df_launch(const PlainCase *pc, const RStage *r, const RApplyArgs &a, int pfrom, int pto) {
   constexpr int T = 128;

@@ -122,14 +122,15 @@ __device__ __forceinline__ void rface(const BlockDev &B, const double *Q, const 
 // k_diffflux, without the flux's round trip between them).  All three axes'
 // faces in one launch, the CTAs of an axis together: no axis waits for the
 // last CTAs of the one before, which on small cases is most of a pass
-template <int NS, int FN, bool VISC>
+template <int NS, int FN, bool KOREN, bool VISC>
 __global__ void __launch_bounds__(RF_TH, 4) k_rface(const BlockDev *__restrict__ blks, const double *__restrict__ Qall,
                                                   const double *__restrict__ stall, const double *__restrict__ trall,
                                                   const double *__restrict__ hall, const double *__restrict__ gall,
                                                   const double *__restrict__ met, double *F0, double *F1, double *F2,
-                                                  const int lim, const int skipu, const unsigned n0, const unsigned n1,
+                                                  const int limiter, const int skipu, const unsigned n0, const unsigned n1,
                                                   const int2 *__restrict__ ctab) {
   constexpr int NE = 4 + NS, NGRAD = NE - 1;
+  const int lim = KOREN ? LIM_KOREN : limiter;
   unsigned t;
   int row;
   const int axis = face_work(n0, n1, ctab, row, t);
@@ -152,11 +153,13 @@ __global__ void __launch_bounds__(RF_TH, 4) k_rface(const BlockDev *__restrict__
 }
 
 // The divergence added to the source (the per-block applyflux's order) and the
-// stage's combines, a component of a cell a thread (the grid's plane the
-// component).  A thread's nine loads are in flight at once and a launch has NE
-// times the threads of a cell-a-thread pass, which walked the components one
-// after another: 64^3 of nine species 65 us and a latency-bound 37 x 29 x 23
-// of the same 32 us that way (ncu).
+// stage's combines, RA_COMPS components of a cell a thread (the grid's plane
+// the group).  A cell a thread walked its components one after another, the
+// loads of each behind the stores of the last: 65 us for 64^3 of nine species
+// and 18 for 53 x 45 x 61 of two; a component a thread spent most of its
+// instructions finding its cell, 42 and 14.7; a group, 40 and 12.5, the first
+// near the 25 its bytes take.
+constexpr int RA_COMPS = 4;
 template <int NS>
 __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blks, int b, const double *__restrict__ Fi,
                                                 const double *__restrict__ Fj, const double *__restrict__ Fk,
@@ -167,33 +170,44 @@ __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blk
   if (t >= (long long)B.nx * B.ny * B.nz) return;
   const long long c = inner_cell(B, t), v = B.vol;
   const long long sJ = B.X, sK = (long long)B.X * B.Y;
-  const long long at = NE * B.cv + (int)blockIdx.z * v + c;
-  const double *fi = Fi + at, *fj = Fj + at, *fk = Fk + at;
+  const int l0 = (int)blockIdx.z * RA_COMPS;
   const double detJinv = B.uniform ? B.detJinv : met[M_NCOMP * B.cv + M_DETJINV * v + c];
   const double dt = *a.dt;
-  double x[2][4];
+  const long long at0 = NE * B.cv + l0 * v + c;
+  double dq[RA_COMPS], first[RA_COMPS];
 #pragma unroll
-  for (int m = 0; m < 2; m++)
+  for (int l = 0; l < RA_COMPS; l++) {
+    if (l0 + l >= NE) break;
+    const long long at = at0 + l * v;
+    const double *fi = Fi + at, *fj = Fj + at, *fk = Fk + at;
+    const double f = fi[0] + fj[0] + fk[0] - fi[1] - fj[sJ] - fk[sK];
+    dq[l] = a.chem ? div_onto(a.dQ[at], f, detJinv) : div_begin(f, detJinv);
+  }
+  if (a.write_dq) {
 #pragma unroll
-    for (int n = 0; n < 4; n++)
-      x[m][n] = m < a.ncomb && n < a.comb[m].nterms && a.comb[m].src[n] >= 0 ? a.comb[m].X[n][at] : 0.0;
-  const double src = a.chem ? a.dQ[at] : 0.0;
-  const double f = fi[0] + fj[0] + fk[0] - fi[1] - fj[sJ] - fk[sK];
-  const double dq = a.chem ? div_onto(src, f, detJinv) : div_begin(f, detJinv);
-  if (a.write_dq) a.dQ[at] = dq;
-  double first = 0.0;
-#pragma unroll
-  for (int m = 0; m < 2; m++) {
-    if (m >= a.ncomb) break;
+    for (int l = 0; l < RA_COMPS; l++)
+      if (l0 + l < NE) a.dQ[at0 + l * v] = dq[l];
+  }
+  for (int m = 0; m < a.ncomb; m++) {
     const RCombine &cb = a.comb[m];
-    auto val = [&](const int n) { return cb.src[n] == -1 ? dq : cb.src[n] == -2 ? first : x[m][n]; };
-    auto weight = [&](const int n) { return term_weight(cb.w[n], cb.step && n == cb.nterms - 1, dt); };
-    double acc = term_first(weight(0), val(0));
+    double acc[RA_COMPS];
+    for (int n = 0; n < cb.nterms; n++) {
+      const double w = term_weight(cb.w[n], cb.step && n == cb.nterms - 1, dt);
+      const int src = cb.src[n];
+      const double *X = cb.X[n];
 #pragma unroll
-    for (int n = 1; n < 4; n++)
-      if (n < cb.nterms) acc = term_next(acc, weight(n), val(n));
-    if (m == 0) first = acc;
-    if (cb.write) cb.out[at] = acc;
+      for (int l = 0; l < RA_COMPS; l++) {
+        if (l0 + l >= NE) break;
+        const double x = src == -1 ? dq[l] : src == -2 ? first[l] : X[at0 + l * v];
+        acc[l] = n == 0 ? term_first(w, x) : term_next(acc[l], w, x);
+      }
+    }
+#pragma unroll
+    for (int l = 0; l < RA_COMPS; l++) {
+      if (l0 + l >= NE) break;
+      if (m == 0) first[l] = acc[l];
+      if (cb.write) cb.out[at0 + l * v] = acc[l];
+    }
   }
 }
 
