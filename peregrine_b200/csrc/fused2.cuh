@@ -32,6 +32,15 @@
 // start: the planes inside the block in registers, the planes below and
 // above it in shared memory.
 //
+// Shared memory is what the stage waits for more than for warps: with every
+// cell value, gradient and flux read back from it, and the combines' registers
+// staged there, a plane took some 350 wavefronts a warp, twelve warps an SM
+// (384 threads, 24 x 10) took the time of eight in proportion, and the
+// 27-block 128^3 TGV 1.213 ms an RK4 step.  A thread that keeps its own column,
+// reads four of a gradient record's six pairs and two of a gradient
+// neighbour's three, and loads the combines' registers straight takes about
+// 190, and the step 1.129 ms; 64^3 0.204 -> 0.180, 32^3 0.0667 -> 0.0595.
+//
 // Measured and set aside: one barrier a plane, with three plane slots, two
 // gradient planes and two face-flux planes standing in for the second (the
 // gradients of plane k+1 formed before the barrier, plane k+3's values after
@@ -186,20 +195,20 @@ __device__ __forceinline__ void cp_wait() {
 template <int NT, int TW, int TH>
 struct F2L {
   static constexpr int LW1 = TW + 2, LH1 = TH + 2, LN1 = LW1 * LH1;
-  static constexpr int LW2 = TW + 4, LN2 = LW2 * (TH + 4), LNR = 2 * (TW + TH), LNT = TW * TH;
-  static constexpr int RAW = 5 * (NT + LNR), PRE = 2 * 5 * LNT, SRC = 2 * (NT + LNR);
+  static constexpr int LW2 = TW + 4, LN2 = LW2 * (TH + 4), LNR = 2 * (TW + TH);
+  static constexpr int RAW = 5 * (NT + LNR), SRC = 2 * (NT + LNR);
   static constexpr int GS = 14;  // a gradient record: twelve values and two of padding
   static_assert(LN1 <= NT, "the tile and its ring fit the CTA");
   static_assert(LNR <= NT, "the outer ring fits the CTA");
   __host__ __device__ static constexpr size_t doubles(bool visc) {
-    return (size_t)2 * P_N * LN2 + (visc ? GS * LN1 : 0) + 10 * LN1 + 3 * RAW + 3 * PRE + 2 * SRC;
+    return (size_t)2 * P_N * LN2 + (visc ? GS * LN1 : 0) + 10 * LN1 + 3 * RAW + 2 * SRC;
   }
 };
 
 template <bool VISC, int NT, int MINB, int TW, int TH>
 __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
   using L = F2L<NT, TW, TH>;
-  constexpr int LW1 = L::LW1, LN1 = L::LN1, LW2 = L::LW2, LN2 = L::LN2, LNR = L::LNR, LNT = L::LNT;
+  constexpr int LW1 = L::LW1, LN1 = L::LN1, LW2 = L::LW2, LN2 = L::LN2, LNR = L::LNR;
   extern __shared__ double smem[];
   __shared__ int s_tile;
   const int tid = threadIdx.x;
@@ -208,8 +217,7 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
   double *Fi = G + (VISC ? L::GS * LN1 : 0);
   double *Fj = Fi + 5 * LN1;
   double *raw = Fj + 5 * LN1;  // [3][5][NT] own cells then [5][LNR] ring cells, per slot
-  double *pre = raw + 3 * L::RAW;  // [3][2][5][LNT]
-  const double **src = reinterpret_cast<const double **>(pre + 3 * L::PRE);  // [2][NT + LNR]
+  const double **src = reinterpret_cast<const double **>(raw + 3 * L::RAW);  // [2][NT + LNR]
   int *svol = reinterpret_cast<int *>(src + L::SRC), *splane = svol + L::SRC;
   for (;;) {
     if (tid == 0) s_tile = (int)atomicAdd(a.counter, 1u);
@@ -244,7 +252,6 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
     const int c1 = ii + LW1 * jj;
     const int c2 = (ii + 1) + LW2 * (jj + 1);
     const bool tile = col && ii >= 1 && ii <= tw && jj >= 1 && jj <= th;
-    const int tc = (ii - 1) + tw * (jj - 1);  // this tile cell's index, for the combine staging
     const bool ring_corner = (ii == 0 || ii == W1 - 1) && (jj == 0 || jj == H1 - 1);
     const bool gcol = col && !ring_corner;
     int r2 = -1, x2 = 0, y2 = 0;
@@ -297,12 +304,20 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
       const double2 *Ps = reinterpret_cast<const double2 *>(P + s * P_N * LN2 + P_N * r);
       const double2 a = Ps[0], b = Ps[1], d = Ps[2];
       CellP c;
-      c.rho = a.x, c.u = a.y, c.v = b.x, c.w = b.y, c.T = d.x, c.e = d.y;
+      c.u = a.x, c.v = a.y, c.w = b.x, c.T = b.y, c.rho = d.x, c.e = d.y;
+      return c;
+    };
+    // what the gradients read of a neighbour: u, v, w, T alone
+    auto getV = [&](int s, int r) {
+      const double2 *Ps = reinterpret_cast<const double2 *>(P + s * P_N * LN2 + P_N * r);
+      const double2 a = Ps[0], b = Ps[1];
+      CellP c{};
+      c.u = a.x, c.v = a.y, c.w = b.x, c.T = b.y;
       return c;
     };
     auto putP = [&](int s, int r, const CellP &c) {
       double2 *Ps = reinterpret_cast<double2 *>(P + s * P_N * LN2 + P_N * r);
-      Ps[0] = make_double2(c.rho, c.u), Ps[1] = make_double2(c.v, c.w), Ps[2] = make_double2(c.T, c.e);
+      Ps[0] = make_double2(c.u, c.v), Ps[1] = make_double2(c.w, c.T), Ps[2] = make_double2(c.rho, c.e);
     };
     // plane p's Q copies for this thread's cells, into raw slot p mod 3
     const int nzb = B.nz;
@@ -323,32 +338,11 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
         for (int l = 0; l < 5; l++) cp8(rs + 5 * NT + l * LNR + tid, q + l * sv);
       }
     };
-    // plane p's combine registers for a tile cell, into pre slot p mod 3
+    // the registers the combines read, at a tile cell (none: a zero weight
+    // takes a zero)
     const long long cbase = 5 * B.cv + o1;
     const double *pre0 = a.prep[0] ? a.prep[0] + cbase : nullptr;
     const double *pre1 = a.prep[1] ? a.prep[1] + cbase : nullptr;
-    auto fetch_pre = [&](int p) {
-      if (!tile) return;
-      double *ps = pre + ring3(p) * L::PRE + tc;
-      const int z = (p + NG) * sK;
-      if (pre0) {
-#pragma unroll
-        for (int l = 0; l < 5; l++) cp8(ps + l * LNT, pre0 + z + l * v);
-      }
-      if (pre1) {
-#pragma unroll
-        for (int l = 0; l < 5; l++) cp8(ps + (5 + l) * LNT, pre1 + z + l * v);
-      }
-    };
-    // a slot no register fills holds zeros, so its zero weight adds nothing
-    if (!pre1 && tile)
-      for (int q = 0; q < 3; q++)
-#pragma unroll
-        for (int l = 0; l < 5; l++) pre[q * L::PRE + (5 + l) * LNT + tc] = 0.0;
-    if (!pre0 && tile)
-      for (int q = 0; q < 3; q++)
-#pragma unroll
-        for (int l = 0; l < 5; l++) pre[q * L::PRE + l * LNT + tc] = 0.0;
     auto own_raw = [&](int p) {
       const double *rs = raw + ring3(p) * L::RAW + tid;
       return prim_of(rs[0 * NT], rs[1 * NT], rs[2 * NT], rs[3 * NT], rs[4 * NT]);
@@ -357,13 +351,30 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
       const double *rs = raw + ring3(p) * L::RAW + 5 * NT + tid;
       return prim_of(rs[0 * LNR], rs[1 * LNR], rs[2 * LNR], rs[3 * LNR], rs[4 * LNR]);
     };
+    // a cell's gradient record as the faces of its two high neighbours read it:
+    // the i-face four of its six pairs, the j-face four, two of them shared
+    // (u_x stands twice; T_z, the k-face's alone, stays in registers)
     auto putG = [&](const double *g) {
-#pragma unroll
-      for (int q = 0; q < 12; q += 2)
-        reinterpret_cast<double2 *>(G + L::GS * c1)[q / 2] = make_double2(g[q], g[q + 1]);
+      double2 *Gs = reinterpret_cast<double2 *>(G + L::GS * c1);
+      Gs[0] = make_double2(g[9], g[6]);  // T_x w_x
+      Gs[1] = make_double2(g[2], g[0]);  // u_z u_x
+      Gs[2] = make_double2(g[4], g[8]);  // v_y w_z
+      Gs[3] = make_double2(g[3], g[1]);  // v_x u_y
+      Gs[4] = make_double2(g[5], g[0]);  // v_z u_x
+      Gs[5] = make_double2(g[7], g[10]); // w_y T_y
+    };
+    auto getGi = [&](int r, double *g) {
+      const double2 *Gs = reinterpret_cast<const double2 *>(G + L::GS * r);
+      const double2 a = Gs[0], b = Gs[1], c = Gs[2], d = Gs[3];
+      g[9] = a.x, g[6] = a.y, g[2] = b.x, g[0] = b.y, g[4] = c.x, g[8] = c.y, g[3] = d.x, g[1] = d.y;
+    };
+    auto getGj = [&](int r, double *g) {
+      const double2 *Gs = reinterpret_cast<const double2 *>(G + L::GS * r);
+      const double2 a = Gs[2], b = Gs[3], c = Gs[4], d = Gs[5];
+      g[4] = a.x, g[8] = a.y, g[3] = b.x, g[1] = b.y, g[5] = c.x, g[0] = c.y, g[7] = d.x, g[10] = d.y;
     };
     auto grad_col = [&](int s, const CellP &below, const CellP &above, double *g) {
-      grad_u(B, getP(s, c2 - 1), getP(s, c2 + 1), getP(s, c2 - LW2), getP(s, c2 + LW2), below, above, g);
+      grad_u(B, getV(s, c2 - 1), getV(s, c2 + 1), getV(s, c2 - LW2), getV(s, c2 + LW2), below, above, g);
     };
 
     const int k0 = T.k0, k1 = T.k1;
@@ -384,13 +395,11 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
     if (col) putP(slot(k0 - 1), c2, pm1 = own_raw(k0 - 1));
     if (r2 >= 0) putP(slot(k0 - 1), r2, ring_raw(k0 - 1));
     fetch(k0 + 2);
-    fetch_pre(k0);
     cp_commit();
     cp_wait<2>();
     if (col) putP(slot(k0), c2, p0 = own_raw(k0));
     if (r2 >= 0) putP(slot(k0), r2, ring_raw(k0));
     if (k0 + 3 <= k1 + 1) fetch(k0 + 3);
-    if (k0 + 1 < k1) fetch_pre(k0 + 1);
     cp_commit();
     __syncthreads();
     double gbelow[12];
@@ -400,15 +409,12 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
     if (col) putP(slot(k0 + 1), c2, p1 = own_raw(k0 + 1));
     if (r2 >= 0) putP(slot(k0 + 1), r2, ring_raw(k0 + 1));
     __syncthreads();
-    double Fk[5];
-    {
-      double g0[12];
-      if (VISC && gcol) {
-        grad_col(slot(k0), pm1, p1, g0);
-        putG(g0);
-      }
-      if (tile) face_u<2, VISC>(B, pm1, p0, gbelow, g0, Fk);
+    double Fk[5], gr[12];  // the k-face below plane k, the cell's gradients at plane k
+    if (VISC && gcol) {
+      grad_col(slot(k0), pm1, p1, gr);
+      putG(gr);
     }
+    if (tile) face_u<2, VISC>(B, pm1, p0, gbelow, gr, Fk);
     __syncthreads();
     const double dt = *a.dt;
     const double c00 = a.cw[0][0], c01 = a.cw[0][1], c02 = a.cw[0][2] * dt;
@@ -416,94 +422,83 @@ __global__ void __launch_bounds__(NT, MINB) k_fused2(const FusedArgs a) {
     double *const out0 = a.outp[0], *const out1 = a.outp[1];
     const bool wr0 = a.write[0] && out0, wr1 = a.write[1] && out1;
 
-    // in flight at the top of step k: {plane k+2, combine registers of k},
-    // {plane k+3, combine registers of k+1}
+    // in flight at the top of step k: planes k+2 and k+3; p0, p1 the column's
+    // own cells of planes k and k+1
     for (int k = k0; k < k1; k++) {
       const int s0 = slot(k), s1 = slot(k + 1);
-      // 0. the copies of plane k+4 and of plane k+2's combine registers go
-      //    out: their slots held plane k+1 and k-1, used up last step
+      // 0. the copies of plane k+4 go out (their slot held plane k+1, used up
+      //    last step), and the loads of plane k's combine registers, which
+      //    the step's end takes
       if (k + 4 <= k1 + 1) fetch(k + 4);
-      if (k + 2 < k1) fetch_pre(k + 2);
       cp_commit();
-      // 1. this column's low i and j faces at plane k, both in one straight
-      //    run so their arithmetic interleaves; a ring column on the tile's
-      //    high edges computes both and keeps the one the tile needs, the
-      //    rest of the ring (whole warps of it) none
+      double r0[5], r1[5];
+      if (tile) {
+        const int z = (k + NG) * sK;
+#pragma unroll
+        for (int l = 0; l < 5; l++) r0[l] = pre0 ? __ldcs(pre0 + z + l * v) : 0.0;
+#pragma unroll
+        for (int l = 0; l < 5; l++) r1[l] = pre1 ? __ldcs(pre1 + z + l * v) : 0.0;
+      }
+      // 1. this column's low i and j faces at plane k, one after the other; a
+      //    ring column on the tile's high edges computes both and keeps the
+      //    one the tile needs, the rest of the ring (whole warps of it) none
+      double Fa[5], Fb[5];
       if (needi || needj) {
         const int li = ii >= 1 ? 1 : 0, lj = jj >= 1 ? LW1 : 0;
         const int li2 = ii >= 1 ? 1 : 0, lj2 = jj >= 1 ? LW2 : 0;
-        double Fa[5], Fb[5], gli[12], glj[12], gr[12];
-        if (VISC) {
-          const double2 *Gi = reinterpret_cast<const double2 *>(G + L::GS * (c1 - li));
-          const double2 *Gj = reinterpret_cast<const double2 *>(G + L::GS * (c1 - lj));
-          const double2 *Gr = reinterpret_cast<const double2 *>(G + L::GS * c1);
-#pragma unroll
-          for (int q = 0; q < 6; q++) {
-            const double2 x = Gi[q], y = Gj[q], z = Gr[q];
-            gli[2 * q] = x.x, gli[2 * q + 1] = x.y, glj[2 * q] = y.x, glj[2 * q + 1] = y.y;
-            gr[2 * q] = z.x, gr[2 * q + 1] = z.y;
-          }
-        }
-        const CellP me = getP(s0, c2);
-        face_u<0, VISC>(B, getP(s0, c2 - li2), me, gli, gr, Fa);
-        face_u<1, VISC>(B, getP(s0, c2 - lj2), me, glj, gr, Fb);
+        double gl[12];
+        if (VISC) getGi(c1 - li, gl);
+        face_u<0, VISC>(B, getP(s0, c2 - li2), p0, gl, gr, Fa);
         if (needi) {
 #pragma unroll
           for (int l = 0; l < 5; l++) Fi[l * LN1 + c1] = Fa[l];
         }
+        if (VISC) getGj(c1 - lj, gl);
+        face_u<1, VISC>(B, getP(s0, c2 - lj2), p0, gl, gr, Fb);
         if (needj) {
 #pragma unroll
           for (int l = 0; l < 5; l++) Fj[l * LN1 + c1] = Fb[l];
         }
       }
-      // 2. plane k+2 and plane k's combine registers have landed
+      // 2. plane k+2 has landed
       cp_wait<2>();
       CellP p2{}, p2r{};
       if (col) p2 = own_raw(k + 2);
       if (r2 >= 0) p2r = ring_raw(k + 2);
       __syncthreads();
-      // 3. the gradients of plane k+1, the k face above k, dQ and the combines
-      const CellP pk = col ? getP(s0, c2) : CellP{};
-      const CellP pk1 = col ? getP(s1, c2) : CellP{};
+      // 3. plane k+2 takes plane k's slot (past the barrier no face reads it);
+      //    the gradients of plane k+1, the k face above k, dQ and the combines
+      if (col) putP(s0, c2, p2);
+      if (r2 >= 0) putP(s0, r2, p2r);
       double gup[12];
-      if (VISC && gcol) grad_col(s1, pk, p2, gup);
+      if (VISC && gcol) grad_col(s1, p0, p2, gup);
       if (tile) {
-        double Fkh[5], gk[12];
-        if (VISC) {
-          const double2 *Gc = reinterpret_cast<const double2 *>(G + L::GS * c1);
-#pragma unroll
-          for (int q = 0; q < 6; q++) {
-            const double2 x = Gc[q];
-            gk[2 * q] = x.x, gk[2 * q + 1] = x.y;
-          }
-        } else {
-#pragma unroll
-          for (int q = 0; q < 12; q++) gk[q] = 0.0;
-        }
-        face_u<2, VISC>(B, pk, pk1, gk, gup, Fkh);
+        double Fkh[5];
+        face_u<2, VISC>(B, p0, p1, gr, gup, Fkh);
         const double dJ = B.detJinv;
         double dQ[5];
 #pragma unroll
         for (int l = 0; l < 5; l++)
-          dQ[l] = (Fi[l * LN1 + c1] + Fj[l * LN1 + c1] + Fk[l] - Fi[l * LN1 + c1 + 1] - Fj[l * LN1 + c1 + LW1] - Fkh[l]) * dJ;
+          dQ[l] = (Fa[l] + Fb[l] + Fk[l] - Fi[l * LN1 + c1 + 1] - Fj[l * LN1 + c1 + LW1] - Fkh[l]) * dJ;
         // the combines in their fixed form (no branch, no register lookup)
         const long long at = cbase + (k + NG) * sK;
-        const double *pk3 = pre + ring3(k) * L::PRE + tc;
 #pragma unroll
         for (int l = 0; l < 5; l++) {
-          const double p0 = pk3[l * LNT], p1 = pk3[(5 + l) * LNT];
-          const double o0 = c00 * p0 + c01 * p1 + c02 * dQ[l];
-          const double o1v = c10 * p0 + c11 * p1 + c12 * dQ[l] + c13 * o0;
+          const double o0 = c00 * r0[l] + c01 * r1[l] + c02 * dQ[l];
+          const double o1v = c10 * r0[l] + c11 * r1[l] + c12 * dQ[l] + c13 * o0;
           if (wr0) out0[at + l * v] = o0;
           if (wr1) out1[at + l * v] = o1v;
         }
 #pragma unroll
         for (int l = 0; l < 5; l++) Fk[l] = Fkh[l];
       }
-      // 4. plane k+2 takes plane k's slot, the k+1 gradients plane k's
-      if (col) putP(s0, c2, p2);
-      if (r2 >= 0) putP(s0, r2, p2r);
-      if (VISC && gcol) putG(gup);
+      // 4. the k+1 gradients take plane k's place
+      if (VISC && gcol) {
+        putG(gup);
+#pragma unroll
+        for (int q = 0; q < 12; q++) gr[q] = gup[q];
+      }
+      p0 = p1, p1 = p2;
       __syncthreads();
     }
     cp_wait<0>();

@@ -102,6 +102,7 @@ struct HostBlock {
   int bc[6] = {-1, -1, -1, -1, -1, -1};  // a boundary face's entry, -1 for none
   int tw = 0, th = 0, kchunk = 0;
   bool metrics_set[PGB_NMETRICS] = {};
+  bool tile_set = false;  // the caller's tile, not the default
   BlockDev dev{};
 };
 
@@ -173,6 +174,7 @@ struct pgb_case {
 
   int v2_ctas = 1;      // its resident CTAs per SM
   int v2 = 0;           // its instance: threads per CTA, launch bound, tile layout
+  bool v2_auto = true;  // the instance is the default's to choose
   // the uniform stage reads across faces from the neighbours' cells in place
   // of a halo fill: wanted (the default), and whether every face allows it
   bool pull_want = true, pull_faces = false;
@@ -726,33 +728,48 @@ void default_tile2(HostBlock &B, const V2Inst &v, int ksplit) {
   B.kchunk = (B.nz + ksplit - 1) / ksplit;
 }
 
-// The runs the default tiles cut k in: the fewest rounds of CTAs over the
-// device's SMs times the planes a tile marches, its own and the TILE_LEAD it
-// reads before its first (measured with the launch at 2.1 us a plane and 9 us
-// over them: 32^3 in 3 runs 0.130 ms an RK4 step, in 11 0.062, in 16, more
-// tiles than SMs, 0.082; 64^3 in 3 runs 0.263, in 4 0.204, in 5 0.214; the
-// 27-block 128^3 in 1, 2, 3 and 4 runs 1.318, 1.213, 1.317 and 1.321).
+// The default instance and the runs k is cut in: the fewest rounds of CTAs over
+// the device's SMs times the planes a tile marches, its own and the TILE_LEAD
+// it reads before its first (measured with the launch at some 2 us a plane and
+// 9 us over them).  256 threads an SM, 32^3 in 3 runs 0.130 ms an RK4 step, in
+// 11 0.062, in 16, more tiles than SMs, 0.082; 64^3 in 3 runs 0.263, in 4
+// 0.204, in 5 0.214; the 27-block 128^3 in 1, 2, 3 and 4 runs 1.318, 1.213,
+// 1.317 and 1.321.  The 128-thread instance, two CTAs an SM, takes TILE_PAIR a
+// plane when both run and has twice the slots: an inviscid 61 x 75 x 47 in four
+// blocks, 264 tiles in two rounds 0.104 ms an RK3 step, 260 smaller ones in one
+// 0.086.
 constexpr int TILE_LEAD = 4;
-int default_ksplit(const pgb_case *c) {
-  const V2Inst &v = kV2[c->v2];
+constexpr double TILE_PAIR = 1.15;
+void default_choice(const pgb_case *c, int &v2, int &ksplit) {
   int dev = 0, sms = 148, nzmax = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long slots = (long long)sms * v.minb;
   for (const HostBlock &B : c->blocks) nzmax = std::max(nzmax, B.nz);
-  int best = 1;
-  long long least = 0;
-  for (int s = 1; s <= std::min(nzmax, 32); s++) {
-    long long tiles = 0, most = 0;
-    for (const HostBlock &B : c->blocks) {
-      const long long kc = (B.nz + s - 1) / s;
-      tiles += (long long)((B.nx + v.tw - 1) / v.tw) * ((B.ny + v.th - 1) / v.th) * ((B.nz + kc - 1) / kc);
-      most = std::max(most, kc);
+  double least = -1.0;
+  auto consider = [&](int q) {
+    const V2Inst &v = kV2[q];
+    const long long slots = (long long)sms * v.minb;
+    for (int s = 1; s <= std::min(nzmax, 32); s++) {
+      long long tiles = 0, most = 0;
+      for (const HostBlock &B : c->blocks) {
+        const long long kc = (B.nz + s - 1) / s;
+        tiles += (long long)((B.nx + v.tw - 1) / v.tw) * ((B.ny + v.th - 1) / v.th) * ((B.nz + kc - 1) / kc);
+        most = std::max(most, kc);
+      }
+      const double cost = (double)((tiles + slots - 1) / slots * (most + TILE_LEAD)) *
+                          (v.minb > 1 && tiles > sms ? TILE_PAIR : 1.0);
+      if (least < 0.0 || cost < least) least = cost, v2 = q, ksplit = s;
     }
-    const long long cost = (tiles + slots - 1) / slots * (most + TILE_LEAD);
-    if (s == 1 || cost < least) best = s, least = cost;
-  }
-  return best;
+  };
+  const int asked = c->v2;
+  v2 = asked, ksplit = 1;
+  consider(asked);
+  // an instance or a tile the caller set stays
+  bool open = c->v2_auto;
+  for (const HostBlock &B : c->blocks) open = open && !B.tile_set;
+  if (open)
+    for (int q = 0; q < kNV2; q++)
+      if (q != asked && kV2[q].nt <= 256 && kV2[q].tw != 30) consider(q);
 }
 
 bool tile_fits(const pgb_case *c, int tw, int th) {
@@ -764,7 +781,15 @@ int build_tiles(pgb_case *c) {
   std::vector<TileDev> tiles;
   size_t smem = 0;
   const bool visc = c->phys.simulator == PGB_NAVIER_STOKES;
-  const int ksplit = c->use_v2 ? default_ksplit(c) : 1;
+  int ksplit = 1;
+  if (c->use_v2) {
+    int v2 = c->v2;
+    default_choice(c, v2, ksplit);
+    if (v2 != c->v2) {
+      c->v2 = v2;
+      for (auto &B : c->blocks) B.tw = 0;
+    }
+  }
   for (int b = 0; b < (int)c->blocks.size(); b++) {
     HostBlock &B = c->blocks[b];
     if (B.tw <= 0 || !tile_fits(c, B.tw, B.th)) {
@@ -1633,7 +1658,7 @@ int build_bcs(pgb_case *c) {
 
 // Whether the single-species kepaec case (form 1) steps by the fused passes
 // where its grid is not uniform: 64^3 in four blocks, a Navier-Stokes RK4 step
-// 0.46 ms against the general stage kernel's 1.85 ms.  The stage kernel
+// 0.56 ms against the general stage kernel's 1.85 ms.  The stage kernel
 // keeps the cases of few cells, a shard (its gradients come of Q's traded
 // halo) and a case whose passes' arrays do not fit the device beside it.
 bool passes_take(pgb_case *c) {
@@ -2487,16 +2512,20 @@ int pgb_metric_set(pgb_case *c, int blk, int which, const double *host, long cou
   const int X = D.X + (face == 0), Y = D.Y + (face == 1), Z = D.Z + (face == 2);
   const int nc = comps[which];
   if (count != (long)X * Y * Z * nc) return fail(PGB_ERR_ARG, "metric array of the wrong size");
-  // host F order [comp][k][j][i] over the array's own extents; the face
-  // array's last plane (past the last halo cell) is never read and is dropped
-  std::vector<double> dev((size_t)nc * D.vol);
-  for (int q = 0; q < nc; q++)
-    for (int k = 0; k < D.Z; k++)
-      for (int j = 0; j < D.Y; j++)
-        for (int i = 0; i < D.X; i++)
-          dev[(size_t)q * D.vol + cell_index(D, i, j, k)] = host[(((size_t)q * Z + k) * Y + j) * X + i];
-  CK(cudaMemcpy(c->d_met + (size_t)M_NCOMP * D.cv + (size_t)first[which] * D.vol, dev.data(),
-                sizeof(double) * dev.size(), cudaMemcpyHostToDevice));
+  // the host array is F order over its own extents, as the device's: a cell
+  // array copies straight; a face array's rows (i faces), planes (j) or
+  // volumes (k) are one cell longer, and that last cell, past the halo, is
+  // never read: a pitched copy drops it
+  double *dst = c->d_met + (size_t)M_NCOMP * D.cv + (size_t)first[which] * D.vol;
+  const size_t w = sizeof(double);
+  if (face < 0)
+    CK(cudaMemcpy(dst, host, w * nc * D.vol, cudaMemcpyHostToDevice));
+  else if (face == 0)
+    CK(cudaMemcpy2D(dst, w * D.X, host, w * X, w * D.X, (size_t)D.Y * D.Z * nc, cudaMemcpyHostToDevice));
+  else if (face == 1)
+    CK(cudaMemcpy2D(dst, w * D.X * D.Y, host, w * D.X * Y, w * D.X * D.Y, (size_t)D.Z * nc, cudaMemcpyHostToDevice));
+  else
+    CK(cudaMemcpy2D(dst, w * D.vol, host, w * (size_t)D.X * D.Y * Z, w * D.vol, (size_t)nc, cudaMemcpyHostToDevice));
   B.metrics_set[which] = true;
   c->uniform_done = false;
   for (auto &g : c->graph)
@@ -2894,6 +2923,7 @@ int pgb_set_tile(pgb_case *c, int blk, int tw, int th, int kchunk) {
   if (tw == 0 && th == 0) {
     // back to the default tile of the case's kernel
     B.tw = 0;
+    B.tile_set = false;
     c->tiles_dirty = true;
     for (auto &g : c->graph)
       if (g) cudaGraphExecDestroy(g), g = nullptr;
@@ -2901,6 +2931,7 @@ int pgb_set_tile(pgb_case *c, int blk, int tw, int th, int kchunk) {
   }
   if (tw < 1 || th < 1 || kchunk < 1) return fail(PGB_ERR_ARG, "bad tile");
   B.tw = std::min(tw, B.nx), B.th = std::min(th, B.ny), B.kchunk = std::min(kchunk, B.nz);
+  B.tile_set = true;
   c->tiles_dirty = true;
   for (auto &g : c->graph)
     if (g) cudaGraphExecDestroy(g), g = nullptr;
@@ -2911,8 +2942,13 @@ int pgb_get_tile(const pgb_case *c, int blk, int *tw, int *th, int *kchunk) {
   if (!c || blk < 0 || blk >= (int)c->blocks.size() || !tw || !th || !kchunk) return fail(PGB_ERR_ARG, "bad argument");
   HostBlock B = c->blocks[blk];
   if (B.tw <= 0) {
-    if (c->use_v2) default_tile2(B, kV2[c->v2], default_ksplit(c));
-    else default_tile(B);
+    if (c->use_v2) {
+      int v2 = c->v2, ksplit = 1;
+      default_choice(c, v2, ksplit);
+      default_tile2(B, kV2[v2], ksplit);
+    } else {
+      default_tile(B);
+    }
   }
   *tw = B.tw, *th = B.th, *kchunk = B.kchunk;
   return PGB_OK;
@@ -2930,8 +2966,9 @@ int pgb_set_fused_shape(pgb_case *c, int threads, int minblocks, int width) {
     return fail(PGB_ERR_ARG, "no uniform kernel of that shape; threads x minblocks x width:" + have);
   }
   if (pick != c->v2)
-    for (auto &B : c->blocks) B.tw = 0;
+    for (auto &B : c->blocks) B.tw = 0, B.tile_set = false;
   c->v2 = pick;
+  c->v2_auto = false;
   c->tiles_dirty = true;
   for (auto &g : c->graph)
     if (g) cudaGraphExecDestroy(g), g = nullptr;
