@@ -57,12 +57,14 @@ _METRICS = {}
 
 def box_metrics(cells, lengths):
     """The grid metrics of a periodic box (cached by shape and size), from
-    the same mesher and metric code every case uses."""
+    the same mesher and metric code every case uses, in the device's order (i
+    fastest), so an admission hands them over as they are."""
     key = (tuple(cells), tuple(float(x) for x in lengths))
     if key not in _METRICS:
         mesh = CubeMesher(cells=[[c] for c in cells], lengths=list(lengths), periodic=[True] * 3)
         blk = mesh.make_blocks(NG)[0]
-        _METRICS[key] = make_metrics(blk.nodes, NG)
+        _METRICS[key] = {name: np.asfortranarray(a.reshape(a.shape[:3] + (-1,))).reshape(a.shape)
+                         for name, a in make_metrics(blk.nodes, NG).items()}
     return _METRICS[key]
 
 
