@@ -2518,14 +2518,19 @@ int pgb_metric_set(pgb_case *c, int blk, int which, const double *host, long cou
   // never read: a pitched copy drops it
   double *dst = c->d_met + (size_t)M_NCOMP * D.cv + (size_t)first[which] * D.vol;
   const size_t w = sizeof(double);
+  // on the case's stream, before the launches that will read it, and waited
+  // for: a page-locked array is the caller's again when the call returns
   if (face < 0)
-    CK(cudaMemcpy(dst, host, w * nc * D.vol, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(dst, host, w * nc * D.vol, cudaMemcpyHostToDevice, c->stream));
   else if (face == 0)
-    CK(cudaMemcpy2D(dst, w * D.X, host, w * X, w * D.X, (size_t)D.Y * D.Z * nc, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy2DAsync(dst, w * D.X, host, w * X, w * D.X, (size_t)D.Y * D.Z * nc, cudaMemcpyHostToDevice, c->stream));
   else if (face == 1)
-    CK(cudaMemcpy2D(dst, w * D.X * D.Y, host, w * D.X * Y, w * D.X * D.Y, (size_t)D.Z * nc, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy2DAsync(dst, w * D.X * D.Y, host, w * D.X * Y, w * D.X * D.Y, (size_t)D.Z * nc, cudaMemcpyHostToDevice,
+                         c->stream));
   else
-    CK(cudaMemcpy2D(dst, w * D.vol, host, w * (size_t)D.X * D.Y * Z, w * D.vol, (size_t)nc, cudaMemcpyHostToDevice));
+    CK(cudaMemcpy2DAsync(dst, w * D.vol, host, w * (size_t)D.X * D.Y * Z, w * D.vol, (size_t)nc, cudaMemcpyHostToDevice,
+                         c->stream));
+  CK(cudaStreamSynchronize(c->stream));
   B.metrics_set[which] = true;
   c->uniform_done = false;
   for (auto &g : c->graph)

@@ -1,0 +1,42 @@
+"""The double flux's batched stages with p handed from stage to stage
+(df_stage, csrc/pgb_host.cu; k_rcellflux_df, csrc/react.cuh) against the
+per-block path: thin blocks, whose state is formed on the interior and copied,
+and a thick one, formed over the halo too; the integrators' stage counts, with
+two, three and four stages p's two fields taken in turn.
+
+The bar is the per-block path's of the other batched tests: rounding, 1e-12 of
+each component's largest."""
+
+import numpy as np
+import pytest
+
+from peregrine_b200 import cases, native
+
+pytestmark = pytest.mark.gpu
+
+
+def layer(launch, integrator, mesh):
+    import peregrine_b200 as pg
+
+    cfg = cases.mixing_layer_config("pr", "euler-df", integrator, launch)
+    mb = pg.get_solver(cfg, cases.mixing_layer_mesh(*mesh), pg.get_backend("cuda", cfg))
+    mb.set_prims(cases.mixing_layer_prims(mb.metrics, mesh[1], seed=2))
+    return mb
+
+
+@pytest.mark.parametrize("mesh", [(37, 31, 3, 2), (48, 48, 48, 1)])
+@pytest.mark.parametrize("integrator", ["rk1", "rk2", "tvd-rk3", "rk4", "rk34"])
+def test_steps_as_the_per_block_path(mesh, integrator):
+    a, b = layer("batched", integrator, mesh), layer("per-block", integrator, mesh)
+    assert a.path == native.PATH_BATCHED and a.batched_form() == 2
+    for mb in (a, b):
+        mb.step(1e-9, 3)
+    for x, y in zip(a.blocks, b.blocks):
+        got, want = x.Q.get()[x.mesh.interior], y.Q.get()[y.mesh.interior]
+        scale = np.abs(want).reshape(-1, want.shape[-1]).max(axis=0)
+        scale[1:4] = scale[1:4].max()
+        assert (np.abs(got - want).reshape(-1, want.shape[-1]).max(axis=0) / scale).max() < 1e-12
+        # the state the last stage's right-hand side formed
+        for name in ("p", "T"):
+            got, want = (mb.sim.iovars.data(blk, [name])[name][x.mesh.interior] for mb, blk in ((a, x), (b, y)))
+            assert np.abs(got - want).max() < 1e-9 * np.abs(want).max()
