@@ -367,7 +367,9 @@ int pgb_set_prims(pgb_case *c, int blk, int reg, const double *host, long count)
 int pgb_rhs(pgb_case *c, int q, int dq);
 /* The same right-hand side on a chosen path (the reference's Solver.rhs,
  * peregrine/multiblock/solver.py:270-273): PGB_PATH_PER_BLOCK as pgb_rhs,
- * PGB_PATH_PACKED the same kernels one launch a pass, PGB_PATH_BATCHED the
+ * PGB_PATH_PACKED the same kernels one launch a pass (a bounded ideal-gas case
+ * of 2048 cells or more whose blocks are all uniform forms its faces as the
+ * batched path's uniform faces do, the same to rounding), PGB_PATH_BATCHED the
  * fused stage kernel itself with one combine dQ = 1 x dt x dQ at dt = 1 (the
  * halo fill of q, then one launch; PGB_ERR_UNSUPPORTED for a case the fused
  * kernel does not take).  The batched form keeps no eos state array.
@@ -446,8 +448,8 @@ int pgb_case_halo_pull(const pgb_case *c, int *on);
  * calorically perfect single-species gas with kepaec on the cells as they
  * are), 2 the fused passes (any other ideal gas, flux function and
  * reconstruction, inviscid or viscous, with or without the coupled
- * chemistry: a cell pass and one tile kernel of every face, the divergence
- * and the combines a stage), 0 neither (boundaries, the real gas, the double
+ * chemistry: a cell pass, the faces, the divergence with the combines; form 1
+ * steps by them too where its grid is not uniform), 0 neither (boundaries, the real gas, the double
  * flux, the sub-stepped chemistry run the per-block kernels, packed).  No
  * counterpart in the reference, whose every case runs its per-kernel launches
  * (peregrine/simulator/advecdiff/simulator.py:110-124). */

@@ -1,19 +1,24 @@
 // The fused passes: one right-hand side and Runge-Kutta stage of the general
 // gas (one to twelve species, calorically or thermally perfect, any flux
 // function and reconstruction, inviscid or viscous, coupled chemistry) in
-// six to eight launches over every block instead of the per-block path's
+// four to seven launches over every block instead of the per-block path's
 // fourteen:
 //
-//   k_rcell   per cell, halo included: fromQ (the eos's Newton from the
-//             cell's last T), then the transport properties and species
-//             enthalpies (the per-block path's k_fromQ then k_transport, one
-//             thread doing both on the state it just formed)
+//   k_rcell   per interior cell: fromQ (the eos's Newton from the cell's last
+//             T), then the transport properties and species enthalpies (the
+//             per-block path's k_fromQ then k_transport, one thread doing both
+//             on the state it just formed)
 //             (peregrine/simulator/euler/kernels/state/fromQ.mako:5-19,
 //              peregrine/simulator/navstokes/kernels/transport.mako:5-35);
+//   k_halo_fields  Q's halo and every field's, in one pass over the halo's
+//             boxes (uniface.cuh); a shard, whose traded halo cells get Q
+//             alone, fills Q's first and forms the cells over the halo too;
 //   k_source  the coupled chemistry source beginning dQ, as on the per-block
 //             path (peregrine/simulator/chemint/kernels/source.mako:3-10);
-//   k_grads   the cell gradients, then their first halo layer;
-//   k_rface   per axis, one face a thread: the advective flux and the
+//   k_ufaces  uniform blocks: the faces of all three axes, without gradient
+//             arrays (uniface.cuh);
+//   k_grads, k_rface  the other blocks: the cell gradients and their first
+//             halo layer, then one face a thread, the advective flux and the
 //             diffusive rows in the same thread, stored once (the per-block
 //             path stores the advective flux, then reads and stores it again
 //             with the diffusive rows added);
@@ -22,9 +27,9 @@
 //             (peregrine/simulator/advec/kernels/applyflux.mako:2-11,
 //              peregrine/integrators/kernels/combine.mako:1-13).
 //
-// Each face and cell runs the per-block kernels' own device functions in the
-// same order; the two paths' results agree to the rounding of the multiply-
-// adds the compiler contracts differently in the two kernels.
+// The cells and the general faces run the per-block kernels' own device
+// functions in the same order, the uniform faces the same arithmetic without
+// its zeros; the two paths' results agree to rounding.
 //
 // Measured and set aside: (a) the chemistry source in the cell kernel, the
 // rate state then spilling to local memory, 0.80 ms a pass at 96^3 against
@@ -36,7 +41,8 @@
 // launch ordered slab by slab, so a slab's cell records are read by all its
 // faces while in L2: 5.3 to 5.8 ms an RK3 step over slabs of 2 to 96 planes
 // against 5.4 ms for the passes per axis (the face passes wait on load
-// latency, not on DRAM bandwidth).
+// latency, not on DRAM bandwidth); the plain axis-after-axis launch kept here
+// saves the two tails, which small cases feel.
 #pragma once
 #include "chem.cuh"
 #include "layout.cuh"
