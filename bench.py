@@ -279,8 +279,8 @@ def reacting_leg(steps, cpu=True):
     out = {"value": b["value"], "unit": "cell-stage/s", "steps": steps, "ms_per_step": b["ms_per_step"],
            "launches_per_step": b["launches_per_step"], "dt": dt,
            "workload": "h2-air-96^3-9sp-28rxn-tpg-kinetic-coupled-chem-muscl-koren-hllc-ns-tvd-rk3",
-           "path": "batched: the fused passes (cell pass, source, gradients, a face pass per axis with the "
-                   "advective and diffusive flux in one thread, divergence and combines in one pass)",
+           "path": "batched: the fused passes (cell pass, every field's halo, source, the faces of all three axes "
+                   "in one launch without gradient arrays, divergence and combines in one pass)",
            "per_block": legs["per_block"], "packed": legs["packed"],
            "speedup_vs_per_block": legs["per_block"]["ms_per_step"] / b["ms_per_step"],
            "batched_launch_kinds": share,
@@ -309,8 +309,8 @@ def reacting_leg(steps, cpu=True):
 def reacting_profile(kernel):
     """The reacting case's batched step twice (a warm-up and one more), its
     launches plain (no graph), so a profiler sees each pass on its own: the
-    stage's seven launches after a halo fill (cell pass, source, gradients,
-    gradient halo, three face passes, divergence and combines)."""
+    stage's five launches (cell pass, every field's halo, source, faces,
+    divergence and combines)."""
     import peregrine_b200 as pg
     from peregrine_b200 import cases
 
@@ -446,9 +446,9 @@ def realgas_leg(steps, cpu=True):
     out = {"value": b["value"], "unit": "cell-stage/s", "steps": steps, "ms_per_step": b["ms_per_step"],
            "launches_per_step": b["launches_per_step"], "dt": dt,
            "workload": "mixing-layer-256x128x4-8-uneven-blocks-o2-h2-60bar-peng-robinson-double-flux-kepaec-euler-rk3",
-           "path": "batched: the planes frozen each step (a launch a pass over every block), then per stage the "
-                   "interior's state off the planes, Q's halo with the state's copy in one pass, and one kernel "
-                   "of each cell's six faces, divergence and combines",
+           "path": "batched: the planes frozen each step (a launch a pass over every block), then per stage "
+                   "Q's and p's halo and one kernel of each cell's six faces, divergence, combines and the next "
+                   "stage's p; the whole state in the last stage",
            "blocks": [b_.cells[0] for b_ in mb.mesh_blocks], "per_block": legs["per_block"], "packed": legs["packed"],
            "speedup_vs_per_block": legs["per_block"]["ms_per_step"] / b["ms_per_step"],
            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,

@@ -492,10 +492,10 @@ extern "C" int PGB_ENTRY(pgb_plain_prestep_)(const PlainCase *pc, double *Q, int
   return e == cudaSuccess ? PGB_OK : cuda_fail(e, "double-flux freeze");
 }
 
-// The fused passes' stage (react.cuh): Q's halo, the cell pass (fromQ, the
-// transport and the coupled source), the gradients and their first halo
-// layer, and the tile kernel (every face, the divergence and the combines),
-// each pass one launch over every block
+// The fused passes' stage (react.cuh): the cell pass (fromQ and the transport),
+// Q's halo and every field's, the coupled source, the faces (the blocks that
+// are not uniform after their gradients and the gradients' halo) and the
+// divergence with the combines, each pass one launch over every block
 namespace {
 template <bool VISC>
 void rcell_launch(const PlainCase *pc, int b, dim3 g, const int2 *ct, const void *ctx) {
