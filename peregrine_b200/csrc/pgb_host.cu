@@ -1276,27 +1276,39 @@ bool passes(const pgb_case *c) { return c->form == 2 || (c->form == 1 && c->by_p
 // stage forms the whole state (the next step's first guess of T, and what
 // pgb_eos_get reads); the first takes p and the halos as the step's start left
 // them.  256 x 128 x 4 cells in 8 blocks, an RK3 step 0.16 ms against 0.202 ms
-// with a state pass and a halo pass of every field each stage.  stage -1: a
-// right-hand side alone.
-void df_stage(const pgb_case *c, const FusedStagePlan &p, int stage, RStage &r) {
+// with a state pass and a halo pass of every field each stage.  A stage leaves
+// p where one of its combines is the register the next stage reads; past a
+// stage whose combines are not (the table reads a register again), each forms
+// its own state.  stage -1: a right-hand side alone.
+void df_stage(const pgb_case *c, int stage, RStage &r) {
   r.full = 1, r.pto = r.pm = -1;
   if (stage < 0 || !sim_df(c->phys.simulator) || c->interior_cells < FEW_CELLS) return;
   const auto &plan = c->plans[c->phase];
   const int last = (int)plan.size() - 1;
+  // the combine of stage s that stage s + 1 reads, -1 for none
+  auto hands = [&](int s) {
+    int pm = -1;
+    for (int m = 0; m < plan[s].ncomb; m++)
+      if (plan[s].comb[m].out == plan[s + 1].qin) pm = m;
+    return pm;
+  };
+  if (stage == last) return;
+  for (int s = 0; s < stage; s++)
+    if (hands(s) < 0) return;
   auto field = [](int s) { return s % 2 ? ST_P2 : 0; };
-  r.full = stage == last;
+  r.full = 0;
   r.pfrom = field(stage);
   r.filled = stage == 0;
   if (stage + 1 >= last) return;
-  for (int m = 0; m < p.ncomb; m++)
-    if (p.comb[m].out == plan[stage + 1].qin) r.pto = field(stage + 1), r.pm = m;
+  r.pm = hands(stage);
+  if (r.pm >= 0) r.pto = field(stage + 1);
 }
 
 // one stage of the fused passes (react.cuh): the plan's combines on physical
 // registers; with dq set (a right-hand side alone) no combine, dQ stored there
 int launch_react(pgb_case *c, const FusedStagePlan &p, int &count, int dq = -1, int stage = -1) {
   RStage r{};
-  df_stage(c, p, stage, r);
+  df_stage(c, stage, r);
   r.Q = c->d_reg[p.qin];
   r.dQ = c->d_reg[dq >= 0 ? dq : p.dqbuf];
   r.write_dq = dq >= 0;

@@ -40,3 +40,45 @@ def test_steps_as_the_per_block_path(mesh, integrator):
         for name in ("p", "T"):
             got, want = (mb.sim.iovars.data(blk, [name])[name][x.mesh.interior] for mb, blk in ((a, x), (b, y)))
             assert np.abs(got - want).max() < 1e-9 * np.abs(want).max()
+
+
+def records(nregs, rows):
+    """Stage records of rows (register read, [(out, own weight, [(register, weight)], dQ's weight)]), dQ the last
+    register."""
+    recs = (native.Stage * len(rows))()
+    for rec, (q, combines) in zip(recs, rows):
+        rec.q, rec.dq, rec.ncombine = q, nregs - 1, len(combines)
+        for cb, (out, own, reads, wdq) in zip(rec.combine, combines):
+            cb.out, cb.own, cb.wout, cb.nterms, cb.step = out, int(own != 0.0), own, len(reads) + 1, 1
+            for n, (r, w) in enumerate(reads + [(-1, wdq)]):
+                cb.reg[n], cb.w[n] = r, w
+    return recs, nregs
+
+
+# tables whose stages do not all read what the stage before wrote: start 0, stages 1 and 2, dQ 3
+REREAD = {
+    # stage 2 reads the register stage 0 wrote
+    "an older stage": [(0, [(1, 0.0, [(0, 1.0)], 0.5)]), (1, [(2, 0.0, [(0, 1.0)], 0.5)]),
+                       (1, [(2, 0.5, [(0, 0.5)], 0.25)]), (2, [(0, 0.5, [(2, 0.5)], 0.5)])],
+    # stage 1 reads the step's start again, and two stages more follow it
+    "the step's start": [(0, [(1, 0.0, [(0, 1.0)], 0.5)]), (0, [(2, 0.0, [(1, 1.0)], 0.25)]),
+                         (2, [(1, 0.0, [(0, 0.75), (2, 0.25)], 0.25)]), (1, [(2, 0.0, [(1, 1.0)], 0.25)]),
+                         (2, [(0, 0.5, [(2, 0.5)], 0.25)])],
+}
+
+
+@pytest.mark.parametrize("mesh", [(37, 31, 3, 2), (48, 48, 48, 1)])
+@pytest.mark.parametrize("table", list(REREAD))
+def test_a_table_that_reads_a_register_again(monkeypatch, mesh, table):
+    from peregrine_b200 import solver
+
+    monkeypatch.setattr(solver, "stage_records", lambda name: records(4, REREAD[table]))
+    a, b = layer("batched", "rk4", mesh), layer("per-block", "rk4", mesh)
+    assert a.path == native.PATH_BATCHED and a.batched_form() == 2
+    for mb in (a, b):
+        mb.step(1e-9, 3)
+    for x, y in zip(a.blocks, b.blocks):
+        got, want = x.Q.get()[x.mesh.interior], y.Q.get()[y.mesh.interior]
+        scale = np.abs(want).reshape(-1, want.shape[-1]).max(axis=0)
+        scale[1:4] = scale[1:4].max()
+        assert (np.abs(got - want).reshape(-1, want.shape[-1]).max(axis=0) / scale).max() < 1e-12
