@@ -1395,9 +1395,7 @@ int ensure_state(pgb_case *c) {
   return PGB_OK;
 }
 
-int ensure_scratch(pgb_case *c) {
-  RET(ensure_state(c));
-  if (c->d_tr) return PGB_OK;
+int alloc_scratch(pgb_case *c) {
   const int ns = c->phys.ns, ne = c->ne, ngrad = ne - 1;
   const size_t n = (size_t)c->cells;
   CK(cudaMalloc(&c->d_tr, sizeof(double) * (2 + ns) * n));
@@ -1419,6 +1417,26 @@ int ensure_scratch(pgb_case *c) {
     CK(cudaMalloc(&c->d_stiffcells, sizeof(int2) * (size_t)c->subopt.bins * (size_t)c->interior_cells));
   }
   return PGB_OK;
+}
+
+template <class T>
+void give_back(T *&p) {
+  if (p) cudaFree(p);
+  p = nullptr;
+}
+
+// the passes' arrays, all of them or none: a call that finds no room leaves
+// none behind for a later one to take for the whole set
+int ensure_scratch(pgb_case *c) {
+  int rc = ensure_state(c);
+  if (rc == PGB_OK && c->d_tr) return rc;
+  if (rc == PGB_OK) rc = alloc_scratch(c);
+  if (rc == PGB_OK) return rc;
+  give_back(c->d_tr), give_back(c->d_hsp), give_back(c->d_grads);
+  for (double *&F : c->d_F) give_back(F);
+  give_back(c->d_subs), give_back(c->d_stiffhead), give_back(c->d_stiffcells);
+  cudaGetLastError();  // the failure is reported here, not by the next launch's check
+  return rc;
 }
 
 void mark_cb(void *ctx, int kind) {
