@@ -118,6 +118,9 @@ struct FusedStagePlan {
 
 }  // namespace
 
+// whether the device has room for the passes' arrays: not yet looked at, none, or they are there
+enum { ROOM_UNKNOWN = 0, ROOM_NO = 1, ROOM_YES = 2 };
+
 struct pgb_case {
   pgb_physics phys{};
   Species sp{};
@@ -163,6 +166,7 @@ struct pgb_case {
   void *d_uref = nullptr;  // the blocks' first cells' metrics (UniformRef) and where a block differs from them
   int *d_ubad = nullptr;
   bool by_passes = false;  // form 1 stepping by the fused passes (passes_take)
+  int passes_room = ROOM_UNKNOWN;  // whether the device has room for their arrays
   bool use_v2 = false;  // every block uniform: the uniform-metric fused kernel
   int form = 0;         // the batched path's form: 1 the fused stage kernel, 2 the fused passes
   // a shard's exchange with the other ranks' blocks: the cells it packs and
@@ -1690,15 +1694,24 @@ int build_bcs(pgb_case *c) {
 // where its grid is not uniform: 64^3 in four blocks, a Navier-Stokes RK4 step
 // 0.56 ms against the general stage kernel's 1.85 ms.  The stage kernel
 // keeps the cases of few cells, a shard (its gradients come of Q's traded
-// halo) and a case whose passes' arrays do not fit the device beside it.
+// halo) and a case whose passes' arrays the device has no room for.
+//
+// They are 55 doubles a cell beside the case's own 50, so they are taken up to
+// half the memory that is free: another case of the size still finds room.
+// What is free is looked at once for a set of metrics, so that a case steps by
+// the same kernels, to the same bits, whatever else the device holds later.
 bool passes_take(pgb_case *c) {
   if (c->nxsend || c->nxrecv || c->interior_cells < FEW_CELLS) return false;
-  if (c->d_tr) return true;
-  size_t free_b = 0, total_b = 0;
-  if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) return false;
-  const size_t n = (size_t)c->cells, ns = (size_t)c->phys.ns, ne = (size_t)c->ne;
-  const size_t need = sizeof(double) * n * ((c->d_state ? 0 : SW) + 2 + 2 * ns + 3 * (ne - 1) + 3 * ne);
-  return need + ((size_t)1 << 28) < free_b;
+  if (c->passes_room == ROOM_UNKNOWN) {
+    c->passes_room = c->d_tr ? ROOM_YES : ROOM_NO;
+    size_t free_b = 0, total_b = 0;
+    if (!c->d_tr && cudaMemGetInfo(&free_b, &total_b) == cudaSuccess) {
+      const size_t n = (size_t)c->cells, ns = (size_t)c->phys.ns, ne = (size_t)c->ne;
+      const size_t need = sizeof(double) * n * ((c->d_state ? 0 : SW) + 2 + 2 * ns + 3 * (ne - 1) + 3 * ne);
+      if (need <= free_b / 2 && ensure_scratch(c) == PGB_OK) c->passes_room = ROOM_YES;
+    }
+  }
+  return c->passes_room == ROOM_YES;
 }
 
 int prepare(pgb_case *c, bool fused) {
@@ -1725,6 +1738,7 @@ int prepare(pgb_case *c, bool fused) {
     for (auto &B : c->blocks) all = all && B.dev.uniform;
     if (all != c->use_v2) c->tiles_dirty = true;
     c->use_v2 = all;
+    c->passes_room = ROOM_UNKNOWN;
   }
   // a grid of general metrics: the stage kernel reads 31 metric components a
   // cell and is bound by the loads each face waits for; the passes are not

@@ -47,3 +47,37 @@ def test_no_room_and_then_room():
         torch.cuda.empty_cache()
     mb.step(1e-5, 2)
     assert np.array_equal(mb.blocks[0].Q.get(), want.blocks[0].Q.get())
+
+
+def curvilinear(n):
+    import peregrine_b200 as pg
+
+    cfg = cases.tgv_config("navier-stokes", "rk4", "batched")
+    mb = pg.get_solver(cfg, cases.tgv_mesh(n, jostle=0.2), pg.get_backend("cuda", cfg))
+    mb.set_prims(cases.tgv_prims(mb.mesh_blocks, mb.metrics, seed=1, noise=1e-3))
+    return mb
+
+
+def test_a_curvilinear_case_keeps_to_its_kernels():
+    """A single-species case on a general grid steps by the passes where the device has room for their arrays and by
+    the stage kernel where it has not; which is settled by its first step, for graphs and single launches alike."""
+    import torch
+
+    curvilinear(16).step(1e-4, 1)
+    roomy, tight = curvilinear(96), curvilinear(96)
+    roomy.step(1e-4, 2)
+    passes = roomy.launches_per_step()
+    held = fill(128 << 20)  # 250 MB are wanted
+    try:
+        tight.step(1e-4, 1)
+        stage = tight.launches_per_step()
+        assert stage < passes
+        roomy.step(1e-4, 1)
+        assert roomy.launches_per_step() == passes
+    finally:
+        del held
+        torch.cuda.empty_cache()
+    for graph in (True, False):
+        tight.graph = graph
+        tight.step(1e-4, 2)
+        assert tight.launches_per_step() == stage
