@@ -178,7 +178,8 @@ struct pgb_case {
 
   int v2_ctas = 1;      // its resident CTAs per SM
   int v2 = 0;           // its instance: threads per CTA, launch bound, tile layout
-  bool v2_auto = true;  // the instance is the default's to choose
+  int v2_from = 0;      // the instance the caller asked for, or the library's first
+  bool v2_auto = true;  // none was asked for: the default may choose another
   // the uniform stage reads across faces from the neighbours' cells in place
   // of a halo fill: wanted (the default), and whether every face allows it
   bool pull_want = true, pull_faces = false;
@@ -765,7 +766,7 @@ void default_choice(const pgb_case *c, int &v2, int &ksplit) {
       if (least < 0.0 || cost < least) least = cost, v2 = q, ksplit = s;
     }
   };
-  const int asked = c->v2;
+  const int asked = c->v2_from;
   v2 = asked, ksplit = 1;
   consider(asked);
   // an instance or a tile the caller set stays
@@ -787,16 +788,16 @@ int build_tiles(pgb_case *c) {
   const bool visc = c->phys.simulator == PGB_NAVIER_STOKES;
   int ksplit = 1;
   if (c->use_v2) {
-    int v2 = c->v2;
-    default_choice(c, v2, ksplit);
-    if (v2 != c->v2) {
-      c->v2 = v2;
-      for (auto &B : c->blocks) B.tw = 0;
-    }
+    // a set tile runs on the instance asked for (the first, when none was):
+    // one that instance does not hold is replaced, and set no longer
+    c->v2 = c->v2_from;
+    for (auto &B : c->blocks) B.tile_set = B.tile_set && tile_fits(c, B.tw, B.th);
+    default_choice(c, c->v2, ksplit);
   }
   for (int b = 0; b < (int)c->blocks.size(); b++) {
     HostBlock &B = c->blocks[b];
-    if (B.tw <= 0 || !tile_fits(c, B.tw, B.th)) {
+    B.tile_set = B.tile_set && tile_fits(c, B.tw, B.th);
+    if (!B.tile_set) {
       if (c->use_v2) default_tile2(B, kV2[c->v2], ksplit);
       else default_tile(B);
     }
@@ -2971,7 +2972,6 @@ int pgb_set_tile(pgb_case *c, int blk, int tw, int th, int kchunk) {
   HostBlock &B = c->blocks[blk];
   if (tw == 0 && th == 0) {
     // back to the default tile of the case's kernel
-    B.tw = 0;
     B.tile_set = false;
     c->tiles_dirty = true;
     for (auto &g : c->graph)
@@ -2990,9 +2990,9 @@ int pgb_set_tile(pgb_case *c, int blk, int tw, int th, int kchunk) {
 int pgb_get_tile(const pgb_case *c, int blk, int *tw, int *th, int *kchunk) {
   if (!c || blk < 0 || blk >= (int)c->blocks.size() || !tw || !th || !kchunk) return fail(PGB_ERR_ARG, "bad argument");
   HostBlock B = c->blocks[blk];
-  if (B.tw <= 0) {
+  if (!B.tile_set) {
     if (c->use_v2) {
-      int v2 = c->v2, ksplit = 1;
+      int v2 = 0, ksplit = 1;
       default_choice(c, v2, ksplit);
       default_tile2(B, kV2[v2], ksplit);
     } else {
@@ -3014,9 +3014,9 @@ int pgb_set_fused_shape(pgb_case *c, int threads, int minblocks, int width) {
       have += " " + std::to_string(kV2[q].nt) + "x" + std::to_string(kV2[q].minb) + "x" + std::to_string(kV2[q].tw);
     return fail(PGB_ERR_ARG, "no uniform kernel of that shape; threads x minblocks x width:" + have);
   }
-  if (pick != c->v2)
-    for (auto &B : c->blocks) B.tw = 0, B.tile_set = false;
-  c->v2 = pick;
+  if (pick != c->v2_from)
+    for (auto &B : c->blocks) B.tile_set = false;
+  c->v2 = c->v2_from = pick;
   c->v2_auto = false;
   c->tiles_dirty = true;
   for (auto &g : c->graph)
