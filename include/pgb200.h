@@ -420,7 +420,9 @@ int pgb_launches_per_step(const pgb_case *c, int path, int *count);
 
 /* the tile shape the batched kernel uses for blk (set by the autotuner or the
  * caller); tw = th = 0 goes back to the kernel's default.  A tile the case's
- * kernel cannot take is replaced by the default when the work list is built. */
+ * kernel cannot take is replaced by the default when the work list is built.
+ * Tiles and instances are the stage kernel's: a case that steps by the fused
+ * passes (pgb_case_tiled 0) keeps them and runs none. */
 int pgb_set_tile(pgb_case *c, int blk, int tw, int th, int kchunk);
 int pgb_get_tile(const pgb_case *c, int blk, int *tw, int *th, int *kchunk);
 
@@ -454,6 +456,11 @@ int pgb_case_halo_pull(const pgb_case *c, int *on);
  * counterpart in the reference, whose every case runs its per-kernel launches
  * (peregrine/simulator/advecdiff/simulator.py:110-124). */
 int pgb_case_batched_form(const pgb_case *c, int *form);
+
+/* Whether the case's batched steps run the fused stage kernel, which the tiles
+ * and instances above are for (1), or not (0).  A single-species case whose
+ * grid is not uniform settles on it or on the passes at its first batched call. */
+int pgb_case_tiled(const pgb_case *c, int *on);
 
 /* whether blk runs in the uniform-metric form (1) or reads its metric arrays (0) */
 int pgb_block_uniform(const pgb_case *c, int blk, int *uniform);

@@ -45,10 +45,18 @@ def _tiles(mb, threads, ksplit):
 
 
 def tune(mb, dt, steps=3, only=None, ksplits=KSPLITS, verbose=False):
-    """Times every candidate; leaves the fastest set on the case and returns it."""
+    """Times every candidate; leaves the fastest set on the case and returns it.  None where there is nothing to
+    choose: the case's steps run no stage kernel."""
     if mb.path != native.PATH_BATCHED:
         return None
     saved = [b.Q.get() for b in mb.blocks]
+    _time(mb, dt, 1)  # a case's first step settles which kernels it runs
+    tiled = ctypes.c_int()
+    native.call("pgb_case_tiled", mb.case, ctypes.byref(tiled))
+    if not tiled.value:
+        for b, q in zip(mb.blocks, saved):
+            b.Q.set(q)
+        return None
     results = []
     cands = [s[:3] for s in shapes()]
     if only is not None:

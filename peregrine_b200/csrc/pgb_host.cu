@@ -3040,6 +3040,12 @@ int pgb_case_batched_form(const pgb_case *c, int *form) {
   return PGB_OK;
 }
 
+int pgb_case_tiled(const pgb_case *c, int *on) {
+  if (!c || !on) return fail(PGB_ERR_ARG, "null argument");
+  *on = batched_form(c) == 1 && !passes(c);
+  return PGB_OK;
+}
+
 int pgb_block_uniform(const pgb_case *c, int blk, int *uniform) {
   if (!c || blk < 0 || blk >= (int)c->blocks.size() || !uniform) return fail(PGB_ERR_ARG, "bad argument");
   *uniform = c->blocks[blk].dev.uniform;

@@ -255,6 +255,7 @@ SIGNATURES = {
     "pgb_rhs_block_noalloc_max_cells": ([ctypes.c_int], ctypes.c_longlong),
     "pgb_block_uniform": ([ctypes.c_void_p, ctypes.c_int, ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
     "pgb_case_batched_form": ([ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
+    "pgb_case_tiled": ([ctypes.c_void_p, ctypes.POINTER(ctypes.c_int)], ctypes.c_int),
     "pgb_fp64_fma_rate": ([ctypes.POINTER(ctypes.c_double)], ctypes.c_int),
     "pgb_case_halo_entries": ([ctypes.c_void_p, ctypes.c_longlong, ctypes.POINTER(ctypes.c_longlong),
                                ctypes.POINTER(ctypes.c_longlong)], ctypes.c_int),

@@ -54,3 +54,19 @@ def test_an_instance_asked_for_stays():
     mb.step(1e-4, 1)
     assert mb.get_tile(0) == (24, 7, 5)
     assert all(mb.get_tile(b)[0] > 14 for b in range(4))
+
+
+def test_the_tuner_times_the_stage_kernel_alone():
+    import peregrine_b200 as pg
+
+    out = []
+    for jostle in (0.0, 0.2):
+        cfg = cases.tgv_config("navier-stokes", "rk4", "batched")
+        mb = pg.get_solver(cfg, cases.tgv_mesh(24, jostle=jostle), pg.get_backend("cuda", cfg))
+        mb.set_prims(cases.tgv_prims(mb.mesh_blocks, mb.metrics, seed=1, noise=1e-3))
+        inner = mb.blocks[0].mesh.interior
+        before = mb.blocks[0].Q.get()[inner]
+        out.append(autotune.tune(mb, 1e-4, steps=1, ksplits=(1, 2)))
+        assert np.array_equal(mb.blocks[0].Q.get()[inner], before)
+    # a lattice steps by the stage kernel; a grid of general metrics by the passes, which have no tiles
+    assert out[0]["candidates"] == 2 * len(autotune.shapes()) and out[1] is None
