@@ -539,8 +539,8 @@ void ufaces_go(const PlainCase *pc, const RStage *r, int lim) {
   unsigned n[3], rows;
   if (!face_grid(pc, n, rows)) return;
   k_ufaces<NS, FN, KOREN, VISC, TPG><<<dim3(n[0] + n[1] + n[2], rows, 1), UF_TH, 0, pc->stream>>>(
-      pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->bcuni ? pc->grads : nullptr, pc->F[0], pc->F[1], pc->F[2], lim,
-      n[0], n[1], pc->ctab[R_FX]);
+      pc->d_blks, r->Q, pc->state, pc->tr, pc->hsp, pc->bcuni ? pc->grads : nullptr, pc->met, pc->F[0], pc->F[1],
+      pc->F[2], lim, n[0], n[1], pc->ctab[R_FX]);
   mark(pc, 2);
 }
 template <bool VISC, bool TPG>

@@ -177,7 +177,7 @@ __global__ void __launch_bounds__(256) k_rapply(const BlockDev *__restrict__ blk
   const long long c = inner_cell(B, t), v = B.vol;
   const long long sJ = B.X, sK = (long long)B.X * B.Y;
   const int l0 = (int)blockIdx.z * RA_COMPS;
-  const double detJinv = B.uniform ? B.detJinv : met[M_NCOMP * B.cv + M_DETJINV * v + c];
+  const double detJinv = met[M_NCOMP * B.cv + M_DETJINV * v + c];
   const double dt = *a.dt;
   const long long at0 = NE * B.cv + l0 * v + c;
   double dq[RA_COMPS], first[RA_COMPS];
@@ -312,8 +312,9 @@ __global__ void __launch_bounds__(128) k_rcellflux_df(const BlockDev *__restrict
     const long long d = A == 0 ? 1 : A == 1 ? B.X : (long long)B.X * B.Y;
     const long long at = low ? c : c + d;
     double S[3] = {0.0, 0.0, 0.0};
+    // on a uniform block the component along the axis is all of the area
     if (B.uniform) {
-      S[A] = B.S[A];
+      S[A] = M[(M_S + 4 * A) * v + at];
     } else {
 #pragma unroll
       for (int e = 0; e < 3; e++) S[e] = M[(M_S + 3 * A + e) * v + at];
@@ -325,7 +326,7 @@ __global__ void __launch_bounds__(128) k_rcellflux_df(const BlockDev *__restrict
 #pragma unroll
     for (int l = 0; l < NE; l++) acc[l] = f == 0 ? F[l] : low ? acc[l] + F[l] : acc[l] - F[l];
   }
-  const double detJinv = B.uniform ? B.detJinv : M[M_DETJINV * v + c];
+  const double detJinv = M[M_DETJINV * v + c];
   const long long at = NE * B.cv + c;
   const double dt = *a.dt;
   double first[NE], qn[NE];

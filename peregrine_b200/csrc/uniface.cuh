@@ -133,18 +133,23 @@ __device__ __forceinline__ void riemann_axis(const RSide &L, const RSide &R, con
 // st's fields ST_U.. hold the cells' velocities.  gr, when given, holds the
 // cells' velocity gradients (a bounded block's: its halo cells' are set by the
 // boundaries); lo, hi: the low or high cell is a boundary's halo cell whose
-// gradient is the other's.
+// gradient is the other's.  M the block's metrics, of which the face reads its
+// own area: a block is uniform to 1e-12, and its first face's area for every
+// face put that much of p times an area into the momentum, 3.4e-13 of it after
+// five RK3 steps of the 192 x 96 x 96 channel where the face's own leaves
+// 2.7e-14 (against float64 off each cell's own; 14.5 ms for 14.3).
 template <int NS, int A, int FN, bool KOREN, bool VISC, bool TPG>
 __device__ __forceinline__ void uface(const BlockDev &B, const double *__restrict__ Q, const double *__restrict__ st,
                                       const double *__restrict__ tr, const double *__restrict__ hs, const double *__restrict__ gr,
-                                      const bool lo, const bool hi, const int limiter, const long long R, double *__restrict__ Fo, double *sh) {
+                                      const double *__restrict__ M, const bool lo, const bool hi, const int limiter,
+                                      const long long R, double *__restrict__ Fo, double *sh) {
   const int lim = KOREN ? LIM_KOREN : limiter;
   constexpr int B1 = (A + 1) % 3, B2 = (A + 2) % 3;
   const int step[3] = {1, B.X, B.X * B.Y};
   const int d = step[A];
   const long long v = B.vol;
   Q += R, st += R;
-  const double S = B.S[A];
+  const double S = M[(M_S + 4 * A) * v + R];
   double F[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   double rho = 0.0, kor = 0.0;
   const double hJ = 0.5 * B.Jd[A];
@@ -314,7 +319,8 @@ template <int NS, int FN, bool KOREN, bool VISC, bool TPG>
 __global__ void __launch_bounds__(UF_TH, TPG ? 4 : 5) k_ufaces(const BlockDev *__restrict__ blks, const double *__restrict__ Qall,
                                                      const double *__restrict__ stall, const double *__restrict__ trall,
                                                      const double *__restrict__ hall,
-                                                     const double *__restrict__ gall, double *F0, double *F1,
+                                                     const double *__restrict__ gall,
+                                                     const double *__restrict__ met, double *F0, double *F1,
                                                      double *F2, const int lim, const unsigned n0, const unsigned n1,
                                                      const int2 *__restrict__ ctab) {
   constexpr int NE = 4 + NS;
@@ -329,14 +335,14 @@ __global__ void __launch_bounds__(UF_TH, TPG ? 4 : 5) k_ufaces(const BlockDev *_
   const bool lo = pos == 0 && (B.bcg >> (2 * axis) & 1);
   const bool hi = pos == (axis == 0 ? B.nx : axis == 1 ? B.ny : B.nz) && (B.bcg >> (2 * axis + 1) & 1);
   const double *gr = VISC && gall ? gall + 3 * (NE - 1) * B.cv : nullptr;
-  const double *Q = Qall + NE * B.cv, *st = stall + SW * B.cv;
+  const double *Q = Qall + NE * B.cv, *st = stall + SW * B.cv, *M = met + M_NCOMP * B.cv;
   const double *tr = VISC ? trall + (2 + NS) * B.cv : nullptr, *hs = VISC ? hall + NS * B.cv : nullptr;
   const long long at = NE * B.cv;
   __shared__ double flux[VISC ? (NS > 1 ? NS - 1 : 1) * UF_TH : 1];
   double *sh = flux + (VISC ? threadIdx.x : 0);
-  if (axis == 0) uface<NS, 0, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, lo, hi, lim, R, F0 + at, sh);
-  else if (axis == 1) uface<NS, 1, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, lo, hi, lim, R, F1 + at, sh);
-  else uface<NS, 2, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, lo, hi, lim, R, F2 + at, sh);
+  if (axis == 0) uface<NS, 0, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, M, lo, hi, lim, R, F0 + at, sh);
+  else if (axis == 1) uface<NS, 1, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, M, lo, hi, lim, R, F1 + at, sh);
+  else uface<NS, 2, FN, KOREN, VISC, TPG>(B, Q, st, tr, hs, gr, M, lo, hi, lim, R, F2 + at, sh);
 }
 
 // every field the faces read of a halo cell, in one pass over the halo's

@@ -82,3 +82,29 @@ def test_a_table_that_reads_a_register_again(monkeypatch, mesh, table):
         scale = np.abs(want).reshape(-1, want.shape[-1]).max(axis=0)
         scale[1:4] = scale[1:4].max()
         assert (np.abs(got - want).reshape(-1, want.shape[-1]).max(axis=0) / scale).max() < 1e-12
+
+
+def test_each_face_has_its_own_area():
+    """A long block's right-hand side off each face's own area and each cell's own volume (as in
+    test_bounded_uniform_gpu.py): the mass, momentum and species rows as the per-block path's to the rounding of six
+    faces, on a pressure whose differences are its own size.  (The energy row sums a plane's theta p, eps rho and kappa,
+    tens of times their sum each; its bar is the steps' above.)"""
+    import peregrine_b200 as pg
+
+    out = []
+    for launch in ("batched", "per-block"):
+        cfg = cases.mixing_layer_config("pr", "euler-df", "tvd-rk3", launch)
+        mb = pg.get_solver(cfg, cases.mixing_layer_mesh(8, 1500, 7, 1), pg.get_backend("cuda", cfg))
+        prims = cases.mixing_layer_prims(mb.metrics, 1500, seed=2)
+        for q in prims:
+            q[..., 0] *= 1.0 + 0.2 * np.random.default_rng(4).uniform(-1.0, 1.0, q.shape[:-1])
+        mb.set_prims(prims)
+        mb.rhs()
+        out.append(getattr(mb.blocks[0], mb.regs[-1]).get()[mb.blocks[0].mesh.interior])
+        if launch == "batched":
+            assert mb.path == native.PATH_BATCHED and mb.uniform(0)
+    got, want = (x.reshape(-1, x.shape[-1]) for x in out)
+    scale = np.abs(want).max(axis=0)
+    scale[1:4] = scale[1:4].max()
+    err = np.abs(got - want).max(axis=0) / scale
+    assert np.delete(err, 4).max() < 64 * np.finfo(float).eps, err

@@ -91,3 +91,23 @@ def test_uniform_and_curvilinear_blocks_in_one_case():
     a, b = pair(lambda launch: cases.mixing_config("navier-stokes", "tvd-rk3", "hllc", "muscl", "koren", 2, launch),
                 mesh, lambda mb: cases.rough_prims(mb.metrics, 2, seed=3, speed=200.0), 1e-5)
     compare(a, b)
+
+
+def test_each_face_has_its_own_area():
+    """As in test_bounded_uniform_gpu.py: a long block's right-hand side off each face's own area."""
+    import peregrine_b200 as pg
+
+    out = []
+    for launch in ("batched", "per-block"):
+        cfg = cases.mixing_config("euler", "tvd-rk3", "hllc", "muscl", "koren", 2, launch)
+        mb = pg.get_solver(cfg, box((8, 1500, 7), lengths=(0.7, 90.0, 0.7)), pg.get_backend("cuda", cfg))
+        mb.set_prims(cases.bc_box_prims(mb.metrics, 2, seed=3, speed=200.0))
+        mb.rhs()
+        out.append(getattr(mb.blocks[0], mb.regs[-1]).get()[mb.blocks[0].mesh.interior])
+        if launch == "batched":
+            assert mb.path == native.PATH_BATCHED and mb.uniform(0)
+    got, want = (x.reshape(-1, x.shape[-1]) for x in out)
+    scale = np.abs(want).max(axis=0)
+    scale[1:4] = scale[1:4].max()
+    err = (np.abs(got - want).max(axis=0) / scale).max()
+    assert err < 64 * np.finfo(float).eps, err
