@@ -30,6 +30,8 @@ def run(cfg, mesh, prims_of, launch, dt, steps):
 
 
 def compare(a, b, bar=1e-12):
+    # a's packed steps took the uniform faces: its blocks were found uniform, which only they ask for
+    assert a.path == native.PATH_PACKED and all(a.uniform(n) for n in range(len(a.blocks)))
     for x, y in zip(a.blocks, b.blocks):
         for reg in ("Q", a.regs[-1]):
             got, want = getattr(x, reg).get()[x.mesh.interior], getattr(y, reg).get()[y.mesh.interior]
@@ -60,6 +62,39 @@ def test_the_channel(cells, blocks):
         out.append(run(cfg, cases.channel_mesh(cells, blocks),
                        lambda mb: cases.bc_box_prims(mb.metrics, 2, seed=1, speed=30.0), launch, 2e-7, 5))
     compare(*out)
+
+
+@pytest.mark.parametrize("kind", ["no-slp-isot-wall", "mov-adia-wall", "sub-in-fmt", "sub-out-fp"])
+@pytest.mark.parametrize("primary,recon,limiter", [("kepaec", "constant", None), ("hllc", "muscl", "vanleer"),
+                                                   ("rusanov", "muscl", "superbee"), ("ausmup", "muscl", "mc")])
+def test_every_scheme(kind, primary, recon, limiter):
+    out = []
+    for launch in (native.PATH_PACKED, native.PATH_PER_BLOCK):
+        cfg = cases.bc_box_config(kind, ns=3, simulator="navier-stokes", primary=primary, recon=recon,
+                                  limiter=limiter, seed=3)
+        out.append(run(cfg, cases.bc_box_mesh(cells=(14, 13, 13), jostle=0.0),
+                       lambda mb: cases.bc_box_prims(mb.metrics, 3, seed=3, speed=60.0), launch, 2e-7, 3))
+    compare(*out)
+
+
+@pytest.mark.parametrize("kind", ["no-slp-isot-wall", "sub-in-ftptt", "sub-out-fp"])
+@pytest.mark.parametrize("simulator,chemistry", [("euler", False), ("navier-stokes", False), ("navier-stokes", True)])
+@pytest.mark.parametrize("primary,recon,limiter", [("kepaec", "constant", None), ("hllc", "muscl", "koren")])
+def test_thermally_perfect(kind, simulator, chemistry, primary, recon, limiter):
+    """Kinetic-theory transport and the coupled source between the same passes."""
+    if simulator == "euler" and kind.startswith("no-slp"):
+        kind = "slp-isot-wall"
+    out = []
+    for launch in (native.PATH_PACKED, native.PATH_PER_BLOCK):
+        cfg = cases.bc_box_config(kind, simulator=simulator, primary=primary, recon=recon, limiter=limiter, eos="tpg",
+                                  seed=3, tables=cases.H2O2_TABLES)
+        if chemistry:
+            cfg["mixture"]["chemistry"], cfg["chem-integration"]["kind"] = "finite-rate", "coupled"
+            cfg = cfg.validate()
+        out.append(run(cfg, cases.bc_box_mesh(cells=(14, 13, 13), jostle=0.0),
+                       lambda mb: cases.bc_box_prims(mb.metrics, 9, seed=3, speed=60.0), launch, 2e-9, 3))
+    # T's root carries the fits' rounding, as in test_uniform_faces_gpu.py
+    compare(*out, bar=1e-11)
 
 
 @pytest.mark.parametrize("primary,recon,limiter,ns", [("hllc", "muscl", "koren", 2), ("kepaec", "constant", None, 1)])

@@ -56,6 +56,7 @@ def test_calorically_perfect(cells, blocks, primary, recon, limiter):
     for simulator, ns in (("navier-stokes", 3), ("euler", 2)):
         a, b = pair(lambda launch: cases.mixing_config(simulator, "tvd-rk3", primary, recon, limiter, ns, launch),
                     lambda: box(cells, blocks), lambda mb: cases.rough_prims(mb.metrics, ns, seed=3, speed=200.0), 1e-5)
+        assert all(a.uniform(n) for n in range(len(a.blocks)))
         compare(a, b)
 
 
@@ -72,24 +73,30 @@ def test_thermally_perfect(cells, blocks, tables, primary, recon, limiter):
     a, b = pair(lambda launch: cases.reacting_config("navier-stokes", "tvd-rk3", primary, recon, limiter, True, tables,
                                                      launch),
                 lambda: box(cells, blocks, (0.01,) * 3), prims, 2e-8)
+    assert all(a.uniform(n) for n in range(len(a.blocks)))
     # T's root carries the fits' rounding, 1e-13 of T, into the pressure, whose
     # difference across a cell drives a momentum a thousandth of its flux
     compare(a, b, 1e-11)
 
 
-def test_uniform_and_curvilinear_blocks_in_one_case():
-    # a jostled block is read by its metric arrays, a lattice one is not; the
-    # faces between them are formed by both
-    class Half(CubeMesher):
+@pytest.mark.parametrize("simulator", ["euler", "navier-stokes"])
+@pytest.mark.parametrize("primary,recon,limiter", [("hllc", "muscl", "koren"), ("kepaec", "constant", None),
+                                                   ("rusanov", "muscl", "mc")])
+def test_uniform_and_curvilinear_blocks_in_one_case(simulator, primary, recon, limiter):
+    # a jostled block and its neighbours, whose halos hold its nodes, are read
+    # by their metric arrays, the lattice blocks past them are not; the faces
+    # between are formed by both
+    class One(CubeMesher):
         def _shape(self, blk, ijk):
-            self.jostle = 0.1 if ijk[0] else 0.0
+            self.jostle = 0.1 if ijk[0] == 2 else 0.0
             super()._shape(blk, ijk)
 
     def mesh():
-        return Half(mbdims=[2, 1, 1], cells=[[13, 12], [14], [11]], lengths=[2 * np.pi] * 3, periodic=[True] * 3)
+        return One(mbdims=[5, 1, 1], cells=[[7, 6, 5, 4, 6], [14], [11]], lengths=[2 * np.pi] * 3, periodic=[True] * 3)
 
-    a, b = pair(lambda launch: cases.mixing_config("navier-stokes", "tvd-rk3", "hllc", "muscl", "koren", 2, launch),
+    a, b = pair(lambda launch: cases.mixing_config(simulator, "tvd-rk3", primary, recon, limiter, 2, launch),
                 mesh, lambda mb: cases.rough_prims(mb.metrics, 2, seed=3, speed=200.0), 1e-5)
+    assert [a.uniform(n) for n in range(5)] == [True, False, False, False, True]
     compare(a, b)
 
 
