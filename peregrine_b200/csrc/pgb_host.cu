@@ -1249,12 +1249,13 @@ int cfl_prologue(pgb_case *c, int qphys, int &count) {
 }
 
 // a stage's combines on a register table, in place: own first, dQ as
-// src -1, the first combine's value (already in the thread) as src -2
+// src -1, the first combine's value (already in the thread) as src -2, of dQ's
+// own register too once the first combine has written it
 void stage_combines(const pgb_stage &st, double *const *reg, RCombine *out) {
   int written0 = -1;
   auto term = [&](RCombine &rc, int n, int r, double w) {
-    const bool dq = r < 0 || r == st.dq;
-    rc.src[n] = dq ? -1 : r == written0 ? -2 : 0;
+    if (r < 0) r = st.dq;
+    rc.src[n] = r == written0 ? -2 : r == st.dq ? -1 : 0;
     rc.X[n] = rc.src[n] < 0 ? nullptr : reg[r];
     rc.w[n] = w;
   };

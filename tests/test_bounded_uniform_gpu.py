@@ -119,3 +119,27 @@ def test_each_face_has_its_own_area(primary, recon, limiter, ns):
     scale[1:4] = scale[1:4].max()
     err = (np.abs(got - want).max(axis=0) / scale).max()
     assert err < 64 * np.finfo(float).eps, err
+
+
+def test_a_stage_that_scales_its_own_dq(monkeypatch):
+    """A table whose first combine writes dQ's register, which the second then reads: what the combines' own passes
+    read there is the scaled value."""
+    from peregrine_b200 import solver
+
+    def records(name):
+        recs = (native.Stage * 1)()
+        recs[0].q, recs[0].dq, recs[0].ncombine = 0, 1, 2
+        scale, add = recs[0].combine
+        scale.out, scale.nterms, scale.step = 1, 1, 1
+        scale.reg[0], scale.w[0] = -1, 1.0
+        add.out, add.own, add.wout, add.nterms, add.step = 0, 1, 1.0, 1, 0
+        add.reg[0], add.w[0] = 1, 0.5
+        return recs, 2
+
+    monkeypatch.setattr(solver, "stage_records", records)
+    out = []
+    for launch in (native.PATH_PACKED, native.PATH_PER_BLOCK):
+        cfg = cases.bc_box_config("slp-adia-wall", ns=2, primary="hllc", recon="muscl", limiter="koren", seed=3)
+        out.append(run(cfg, cases.bc_box_mesh(cells=(14, 13, 13), jostle=0.0),
+                       lambda mb: cases.bc_box_prims(mb.metrics, 2, seed=3, speed=60.0), launch, 2e-7, 3))
+    compare(*out)
