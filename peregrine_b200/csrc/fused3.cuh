@@ -201,7 +201,8 @@ __global__ void __launch_bounds__(NT, MINB) k_fused3(const FusedArgs a) {
     cp_commit();
     cp_wait<0>();
     prim(k0 + 2);
-    fetch(k0 + 3);
+    // (a tile of one plane at a block's top has no plane k0+3 in the block)
+    if (k0 + 3 <= k1 + 1) fetch(k0 + 3);
     cp_commit();
     __syncthreads();
     if (VISC) {

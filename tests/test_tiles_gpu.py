@@ -70,3 +70,35 @@ def test_the_tuner_times_the_stage_kernel_alone():
         assert np.array_equal(mb.blocks[0].Q.get()[inner], before)
     # a lattice steps by the stage kernel; a grid of general metrics by the passes, which have no tiles
     assert out[0]["candidates"] == 2 * len(autotune.shapes()) and out[1] is None
+
+
+@pytest.mark.parametrize("simulator", ["euler", "navier-stokes"])
+@pytest.mark.parametrize("shape", [(256, 1, 24), (256, 1, 30), (128, 2, 14), (512, 1, 14), (512, 1, 16)])
+@pytest.mark.parametrize("cells,kchunk", [((13, 13, 13), 4), ((17, 9, 10), 9), ((23, 15, 7), 1)])
+def test_tiles_of_one_plane(simulator, shape, cells, kchunk):
+    """The tiles of one plane that k's remainder leaves at a block's top: the planes a tile fetches ahead end with
+    the halo, in every instance."""
+    import peregrine_b200 as pg
+    from peregrine_b200.mesher import CubeMesher
+
+    out = []
+    for tiles in (False, True):
+        cfg = cases.tgv_config(simulator, "rk4", "batched")
+        mesh = CubeMesher(cells=[[c] for c in cells], lengths=[2 * np.pi] * 3, periodic=[True] * 3)
+        mb = pg.get_solver(cfg, mesh, pg.get_backend("cuda", cfg))
+        mb.set_prims(cases.tgv_prims(mb.mesh_blocks, mb.metrics, seed=1, noise=1e-3))
+        if tiles:
+            native.call("pgb_set_fused_shape", mb.case, *shape)
+            native.call("pgb_set_tile", mb.case, 0, 0, 0, 1)
+            mb.step(0.0, 1)
+            tw, th, _ = mb.get_tile(0)
+            mb.set_tile(0, tw, th, kchunk)
+        else:
+            mb.step(0.0, 1)
+        mb.step(1e-3, 3)
+        if tiles:
+            assert mb.get_tile(0) == (tw, th, kchunk)
+        out.append(mb.blocks[0].Q.get()[mb.blocks[0].mesh.interior].reshape(-1, 5))
+    scale = np.abs(out[0]).max(axis=0)
+    scale[1:4] = scale[1:4].max()
+    assert (np.abs(out[1] - out[0]).max(axis=0) / scale).max() < 1e-12
