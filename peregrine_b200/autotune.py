@@ -68,6 +68,8 @@ def tune(mb, dt, steps=3, only=None, ksplits=KSPLITS, verbose=False):
                 mb.set_tile(n, tw, th, kc)
             _time(mb, dt, 1)
             ms = _time(mb, dt, steps)
+        except native.PgbCudaError:
+            raise  # the device's own error: no candidate after it would run
         except native.PgbError as e:
             if verbose:
                 print(f"  {threads}x{minb} k/{ksplit}: {e}")
