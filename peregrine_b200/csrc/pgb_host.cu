@@ -1452,11 +1452,13 @@ void mark_cb(void *ctx, int kind) {
 
 // how many of the blocks the uniform faces take (uniface.cuh), and the rest:
 // the ideal gases with kepaec, or a Riemann solver on MUSCL's sides, and with
-// Lewis diffusion where viscous; the other forms' faces read the metric arrays
+// Lewis diffusion where viscous; the other forms' faces read the metric arrays.
+// The uniform faces work every species' coefficient out from the first's, so a
+// first species that does not diffuse (an infinite Lewis number) is not theirs
 void uniform_counts(const pgb_physics &p, const Species &sp, const BlockDev *dev, int n, PlainCase &pc) {
   const bool takes = !sim_df(p.simulator) && (p.eos == PGB_EOS_CPG || p.eos == PGB_EOS_TPG) &&
                      (p.primary == PGB_FLUX_KEPAEC || p.recon == PGB_RECON_MUSCL) &&
-                     !(sim_visc(p.simulator) && sp.binary);
+                     !(sim_visc(p.simulator) && (sp.binary || !std::isfinite(sp.lewis[0])));
   pc.uni = 0;
   for (int b = 0; b < n; b++) pc.uni += takes && dev[b].uniform;
   pc.gen = n - pc.uni;

@@ -118,3 +118,16 @@ def test_each_face_has_its_own_area():
     scale[1:4] = scale[1:4].max()
     err = (np.abs(got - want).max(axis=0) / scale).max()
     assert err < 64 * np.finfo(float).eps, err
+
+
+@pytest.mark.parametrize("still", ["A", "B", "C"])
+def test_a_species_that_does_not_diffuse(still):
+    """An infinite Lewis number: the species' own coefficient is zero, and the others' are what they were."""
+    def cfg_of(launch):
+        cfg = cases.mixing_config("navier-stokes", "tvd-rk3", "hllc", "muscl", "koren", 3, launch)
+        cfg["mixture"]["species"] = {k: dict(v, lewis=np.inf if k == still else v["lewis"])
+                                     for k, v in cfg["mixture"]["species"].items()}
+        return cfg.validate()
+
+    a, b = pair(cfg_of, lambda: box((13, 17, 11)), lambda mb: cases.rough_prims(mb.metrics, 3, seed=3, speed=200.0), 1e-5)
+    compare(a, b)

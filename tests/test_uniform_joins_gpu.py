@@ -115,3 +115,36 @@ def test_the_double_flux_across_a_quarter_turn(n, nk):
                 Pinwheel(n, nk, n * 2e-5), lambda mb: cases.mixing_layer_prims(mb.metrics, n, seed=2), 1e-9,
                 uniform=[True])
     compare(a, b)
+
+
+def bounded(mesh, simulator, primary, recon, limiter):
+    """The packed steps of a box whose k faces are walls against the per-block ones."""
+    import peregrine_b200 as pg
+
+    out = []
+    for launch in (native.PATH_PACKED, native.PATH_PER_BLOCK):
+        cfg = cases.bc_box_config("no-slp-isot-wall" if simulator == "navier-stokes" else "slp-adia-wall", ns=2,
+                                  simulator=simulator, primary=primary, recon=recon, limiter=limiter, seed=3)
+        mb = pg.get_solver(cfg, mesh, pg.get_backend("cuda", cfg))
+        mb.set_prims(cases.bc_box_prims(mb.metrics, 2, seed=3, speed=60.0))
+        mb.path = launch
+        mb.step(2e-7, 3)
+        out.append(mb)
+    assert all(out[0].uniform(n) for n in range(len(out[0].blocks)))
+    compare(*out)
+
+
+@pytest.mark.parametrize("simulator", ["euler", "navier-stokes"])
+@pytest.mark.parametrize("primary,recon,limiter", SCHEMES)
+def test_bounded_blocks_joined_by_a_quarter_turn(simulator, primary, recon, limiter):
+    mesh = Pinwheel(15, 13, 1.0)
+    mesh.periodic[2], mesh.defaultbc = False, "outer"
+    bounded(mesh, simulator, primary, recon, limiter)
+
+
+@pytest.mark.parametrize("S", ["156", "426", "453"])
+@pytest.mark.parametrize("simulator", ["euler", "navier-stokes"])
+def test_a_bounded_block_laid_out_along_other_axes(S, simulator):
+    mesh = Reoriented(S, 1.0)
+    mesh.periodic[2], mesh.defaultbc = False, "outer"
+    bounded(mesh, simulator, "hllc", "muscl", "koren")
