@@ -131,3 +131,16 @@ def test_a_species_that_does_not_diffuse(still):
 
     a, b = pair(cfg_of, lambda: box((13, 17, 11)), lambda mb: cases.rough_prims(mb.metrics, 3, seed=3, speed=200.0), 1e-5)
     compare(a, b)
+
+
+@pytest.mark.parametrize("simulator", ["euler", "navier-stokes"])
+@pytest.mark.parametrize("primary,recon,limiter", [("kepaec", "constant", None), ("hllc", "muscl", "koren"),
+                                                   ("rusanov", "muscl", "superbee"), ("ausmup", "muscl", "vanleer")])
+def test_supersonic_faces(simulator, primary, recon, limiter):
+    # at this speed faces of both signs are supersonic along every axis, where one side's flux is the face's
+    a, b = pair(lambda launch: cases.mixing_config(simulator, "rk2", primary, recon, limiter, 3, launch),
+                lambda: box((13, 17, 11)), lambda mb: cases.rough_prims(mb.metrics, 3, seed=3, speed=1500.0), 2e-6)
+    assert all(a.uniform(n) for n in range(len(a.blocks)))
+    compare(a, b)
+    got, want = a.cflmax(), b.cflmax()
+    assert all(abs(got[k] - want[k]) < 1e-12 * want[k] for k in want)

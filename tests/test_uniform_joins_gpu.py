@@ -87,6 +87,8 @@ def test_a_block_laid_out_along_other_axes(S, simulator, primary, recon, limiter
                 Reoriented(S, 2 * np.pi), lambda mb: cases.rough_prims(mb.metrics, 3, seed=3, speed=200.0), 1e-5,
                 uniform=[True, S in ("156", "426", "453")])
     compare(a, b)
+    got, want = a.cflmax(), b.cflmax()
+    assert all(abs(got[k] - want[k]) < 1e-12 * want[k] for k in want)
 
 
 @pytest.mark.parametrize("S", ["156", "264"])
