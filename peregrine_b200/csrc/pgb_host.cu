@@ -2741,6 +2741,8 @@ static int step_loop(pgb_case *c, int nsteps, int path, int graph) {
     ~Packed() { c->packed = false; }
   } unpack{c};
   c->packed = path == PGB_PATH_PACKED;
+  // a replayed graph's steps too leave the state array behind, or form it
+  if (nsteps > 0) c->state_stale = fused && c->form != 2;
   CK(cudaEventRecord(c->ev0, c->stream));
   int done = 0;
   while (done < nsteps) {
