@@ -451,8 +451,10 @@ int pgb_case_halo_pull(const pgb_case *c, int *on);
  * are), 2 the fused passes (any other ideal gas, flux function and
  * reconstruction, inviscid or viscous, with or without the coupled
  * chemistry: a cell pass, the faces, the divergence with the combines; form 1
- * steps by them too where its grid is not uniform), 0 neither (boundaries, the real gas, the double
- * flux, the sub-stepped chemistry run the per-block kernels, packed).  No
+ * steps by them too where its grid is not uniform and their arrays take no
+ * more than half the free memory), 0 neither (boundaries, the real gas, the
+ * viscous double flux, the sub-stepped chemistry run the per-block kernels,
+ * packed).  No
  * counterpart in the reference, whose every case runs its per-kernel launches
  * (peregrine/simulator/advecdiff/simulator.py:110-124). */
 int pgb_case_batched_form(const pgb_case *c, int *form);

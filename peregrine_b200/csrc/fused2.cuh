@@ -38,8 +38,10 @@
 // (384 threads, 24 x 10) took the time of eight in proportion, and the
 // 27-block 128^3 TGV 1.213 ms an RK4 step.  A thread that keeps its own column,
 // reads four of a gradient record's six pairs and two of a gradient
-// neighbour's three, and loads the combines' registers straight takes about
-// 190, and the step 1.129 ms; 64^3 0.204 -> 0.180, 32^3 0.0667 -> 0.0595.
+// neighbour's three, and loads the combines' registers straight takes some 200
+// (ncu: 25.9 million a launch over the 122,880 planes its warps march, 210
+// each, or 177 with the four planes a tile reads before its first), and the
+// step 1.07 ms; 64^3 0.204 -> 0.180, 32^3 0.0667 -> 0.0595.
 //
 // Measured and set aside: one barrier a plane, with three plane slots, two
 // gradient planes and two face-flux planes standing in for the second (the
@@ -187,7 +189,7 @@ __device__ __forceinline__ void cp_wait() {
 // a cell's twelve contiguous in a record of GS (14 doubles, for the same
 // reason), Fi[5][LN1], Fj[5][LN1]
 // low-face fluxes, raw[3][5][NT + LNR] the Q copies of three planes in
-// flight, pre[3][2][5][LNT] the combines' registers of three planes, and the
+// flight, and the
 // sources of a thread's two fetched cells in the planes below and above the
 // block (those inside it a thread keeps in registers): src[2][NT + LNR]
 // pointers to the source cell's plane 0, then vol[2][NT + LNR] and

@@ -742,7 +742,11 @@ void default_tile2(HostBlock &B, const V2Inst &v, int ksplit) {
 // 1.317 and 1.321.  The 128-thread instance, two CTAs an SM, takes TILE_PAIR a
 // plane when both run and has twice the slots: an inviscid 61 x 75 x 47 in four
 // blocks, 264 tiles in two rounds 0.104 ms an RK3 step, 260 smaller ones in one
-// 0.086.
+// 0.086.  The 30-wide instance is left to the tuner: with a plane of it counted
+// as the 24-wide one's the rounds do not tell where it wins (60^3 0.118 ms for
+// the default's 0.135, 90^3 0.320 for 0.384, 128^3 0.942 for 1.002) from where
+// it loses (64^3 0.174 for 0.152, 96^3 0.465 for 0.417, the 27 blocks 1.151 for
+// 1.073).  The 512-thread ones lost on every size timed, 32^3 to 160^3.
 constexpr int TILE_LEAD = 4;
 constexpr double TILE_PAIR = 1.15;
 void default_choice(const pgb_case *c, int &v2, int &ksplit) {
@@ -1058,7 +1062,11 @@ int build_plans(pgb_case *c) {
 int grid_for(long long n, int threads) { return (int)std::max<long long>(1, (n + threads - 1) / threads); }
 
 // A case of fewer cells keeps the general passes, a fill a field and a launch
-// an axis: its launch list is held by the tests.
+// an axis, for one reason: the tests hold its launch list (exact counts at 1728
+// and 768 cells).  It is the slower list there too: 12^3 of nine reacting
+// species 328 us an RK3 step where the passes above the line take 118, three
+// species 166 and 64, the double flux 81 and 61, a curvilinear single species
+// 235 and 117 an RK4 step, a bounded box 241 and 134.
 constexpr long long FEW_CELLS = 2048;
 
 enum { K_HALO = 0, K_FUSED = 1, K_BLOCK = 2, K_COMBINE = 3 };

@@ -164,8 +164,10 @@ __device__ __forceinline__ void mixmom(YF Y, double &R, double &cp, double &h298
 // the moments of peregrine/simulator/mixture/eos/tpg/model.py:7-9)
 template <int NS, class YF>
 __device__ __forceinline__ void mixmom_tpg(YF Y, double &R, double &h298, double *cc) {
-  // the sums' multiply-adds spelled out: the kernels that form a state then
-  // form the same bits of it, however the compiler arranges each
+  // the sums' multiply-adds spelled out: the kernels that form an ideal gas's
+  // state then form the same bits of it, however the compiler arranges each
+  // (the uniform faces' reconstructed sides, uniface.cuh, and the real gas's
+  // moments, realgas.cuh, are formed in kernels of one arrangement each)
   R = 0.0, h298 = 0.0;
 #pragma unroll
   for (int t = 0; t < MAXT; t++) cc[t] = 0.0;

@@ -149,7 +149,9 @@ class Solver:
             # the batched path takes the ideal gases without boundaries (the
             # fused stage kernel or the fused passes); other physics runs the
             # per-block kernels, still on the device, packed (each pass one
-            # launch over every block, the same bits)
+            # launch over every block, the same bits; a bounded ideal gas of
+            # 2048 cells or more on uniform blocks by the uniform faces, the
+            # same to rounding)
             self.path = native.PATH_PACKED
         if state is None:
             self._uniform_ics()
